@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "evaluator_base.hpp"
+#include "gemm_f64.cuh"
 #include "helmholtz.cuh"
 #include "helmholtz_far.cuh"
 #include "helmholtz_st.cuh"
@@ -161,6 +162,9 @@ struct Evaluator final : EvaluatorBase {
               const std::vector<double>& ut, bool fused, int64_t ybudget_)
         : plan(pl), stream(s), m(m_), gradients(grad), ybudget(ybudget_) {
         timer.stream = s;
+        int dev = 0;
+        CUDA_TRY(cudaGetDevice(&dev));
+        CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
         level.upload(pl.level);
         idx.upload(pl.idx);
         parent.upload(pl.parent);
@@ -210,9 +214,24 @@ struct Evaluator final : EvaluatorBase {
         dp.nsrc = (int64_t)pl.src_perm.size();
         dp.ntgt = (int64_t)pl.tgt_perm.size();
         // tables rounded entry by entry to T (fmm-tables/src/matrix_set.rs:150 cast)
+        // (f64: the same values packed as the tensor path's fragments, gemm_f64.cuh)
         auto up_tab = [](DevBuf& b, const std::vector<double>& t) {
-            std::vector<T> c(t.begin(), t.end());
-            b.upload(c);
+            if constexpr (!kMixed) {
+                using S = GemmF64<P>;
+                const size_t sets = t.size() / ((size_t)NC * NC);
+                std::vector<double> c(sets * S::TABLE);
+                for_chunks(sets, stage_threads(sets * S::TABLE / 32), [&](size_t, size_t d0, size_t d1) {
+                    for (size_t d = d0; d < d1; ++d) {
+                        const double* a = t.data() + d * NC * NC;  // column-major
+                        pack_f64_table<P>(c.data() + d * S::TABLE, 0, 1,
+                                          [&](int n, int k) { return a[(size_t)k * NC + n]; });
+                    }
+                });
+                b.upload(c);
+            } else {
+                std::vector<T> c(t.begin(), t.end());
+                b.upload(c);
+            }
         };
         up_tab(m2l_tab, m2l);
         up_tab(m2m_tab, m2m);
@@ -288,9 +307,7 @@ struct Evaluator final : EvaluatorBase {
             build_p2p_stream();
         }
         close_pairs = nclose;
-        gemm_smem = GemmShape<P, T>::SMEM;
-        if (gemm_smem > 48 * 1024)
-            CUDA_TRY(cudaFuncSetAttribute(m2l_gemm_kernel<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem));
+        gemm_setup<false>();
         // shared memory opt-in beyond 48 KB where a kernel needs it
         size_t exp_smem = sizeof(T) * (NC * 32 + (size_t)m * 32);
         if (exp_smem > 48 * 1024) {
@@ -299,7 +316,41 @@ struct Evaluator final : EvaluatorBase {
         }
     }
 
-    size_t gemm_smem = 0;
+    // The translation products Y[pair] = A_d X[source] of a tile list: f64 on the FP64 tensor
+    // path (gemm_f64.cuh), with a grid of the blocks that fit the device at once; f32, and the
+    // complex f64 form above p = 8 (whose two planes' fragments exceed a thread's registers),
+    // on the SIMT GEMM, a block a tile.
+    template <bool CPLX>
+    static constexpr bool kDmma = !kMixed && GemmF64<P, CPLX>::OK;
+    int gemm_blocks[2] = {0, 0};  // the f64 GEMM's resident blocks (real, complex)
+    template <bool CPLX>
+    void gemm_setup() {
+        if constexpr (kDmma<CPLX>) {
+            using S = GemmF64<P, CPLX>;
+            CUDA_TRY(cudaFuncSetAttribute(gemm_f64_kernel<P, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          S::SMEM));
+            int occ = 0;
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gemm_f64_kernel<P, CPLX>, 32 * S::WARPS,
+                                                                   S::SMEM));
+            gemm_blocks[CPLX] = std::max(1, occ * num_sms / S::SPLIT);
+        } else if (GemmShape<P, T, CPLX>::SMEM > 48 * 1024) {
+            CUDA_TRY(cudaFuncSetAttribute(m2l_gemm_kernel<P, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          GemmShape<P, T, CPLX>::SMEM));
+        }
+    }
+    template <bool CPLX = false>
+    void gemm(const int32_t* td, const int64_t* tb, const int32_t* tn, int64_t nt, const int64_t* pe,
+              const int32_t* ps, const T* tab, const T* x, T* y) {
+        if (nt <= 0) return;
+        if constexpr (kDmma<CPLX>) {
+            using S = GemmF64<P, CPLX>;
+            const dim3 grid(counted((unsigned)std::min<int64_t>(nt, gemm_blocks[CPLX])), S::SPLIT);
+            gemm_f64_kernel<P, CPLX><<<grid, 32 * S::WARPS, S::SMEM, stream>>>(td, tb, tn, nt, pe, ps, m, tab, x, y);
+        } else {
+            m2l_gemm_kernel<P, T, CPLX><<<counted((unsigned)nt), 256, GemmShape<P, T, CPLX>::SMEM, stream>>>(
+                td, tb, tn, pe, ps, m, tab, x, y);
+        }
+    }
 
     ~Evaluator() override {
         if (near_stream) {
@@ -434,9 +485,8 @@ struct Evaluator final : EvaluatorBase {
             }
             return;
         }
-        m2l_gemm_kernel<P, T><<<counted((unsigned)c.s_nt), 256, gemm_smem, stream>>>(
-            ck_s_d.as<int32_t>() + c.s_t0, ck_s_begin.as<int64_t>() + c.s_t0, ck_s_count.as<int32_t>() + c.s_t0,
-            nullptr, ck_pair_src.as<int32_t>() + c.base, m, m2l_tab.as<T>(), M.as<T>(), Y.as<T>());
+        gemm(ck_s_d.as<int32_t>() + c.s_t0, ck_s_begin.as<int64_t>() + c.s_t0, ck_s_count.as<int32_t>() + c.s_t0,
+             c.s_nt, nullptr, ck_pair_src.as<int32_t>() + c.base, m2l_tab.as<T>(), M.as<T>(), Y.as<T>());
     }
     void reduce_chunk(const Chunk& c, int with_l2l, int with_v, int accumulate) {
         reduce_range(c.b0, c.b1, with_l2l, with_v, accumulate);
@@ -567,9 +617,6 @@ struct Evaluator final : EvaluatorBase {
                                           TcTs<P>::SMEM));
             CUDA_TRY(cudaFuncSetAttribute(m2l_tc_kernel<P, false, kTcAlt>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, TcTs<P, false, kTcAlt>::SMEM));
-            int dev = 0;
-            CUDA_TRY(cudaGetDevice(&dev));
-            CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
         }
     }
 
@@ -1173,10 +1220,8 @@ struct Evaluator final : EvaluatorBase {
     void m2m_level(int l) {  // parents on level l from their children on level l + 1
         const int64_t t0 = m2m_tiles[l], nt = m2m_tiles[l + 1] - m2m_tiles[l];
         const int64_t n = m2m_start[l + 1] - m2m_start[l];
-        if (nt)
-            m2l_gemm_kernel<P, T><<<counted((unsigned)nt), 256, gemm_smem, stream>>>(
-                oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0, oct_tile_count.as<int32_t>() + t0,
-                oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(), m, m2m_tab.as<T>(), M.as<T>(), Yo.as<T>());
+        gemm(oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0, oct_tile_count.as<int32_t>() + t0, nt,
+             oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(), m2m_tab.as<T>(), M.as<T>(), Yo.as<T>());
         if (n)
             m2m_reduce_kernel<P, T><<<counted((unsigned)n), round32(NC), 0, stream>>>(
                 dp, m2m_par.as<int32_t>() + m2m_start[l], n, m, Yo.as<T>(), M.as<T>());
@@ -1227,18 +1272,14 @@ struct Evaluator final : EvaluatorBase {
         const DevBuf& td = l < 0 ? tile_d : ltile_d;
         const DevBuf& tb = l < 0 ? tile_begin : ltile_begin;
         const DevBuf& tn = l < 0 ? tile_count : ltile_count;
-        if (nt)
-            m2l_gemm_kernel<P, T><<<counted((unsigned)nt), 256, gemm_smem, stream>>>(
-                td.as<int32_t>() + t0, tb.as<int64_t>() + t0, tn.as<int32_t>() + t0, nullptr,
-                pair_src.as<int32_t>(), m, m2l_tab.as<T>(), M.as<T>(), Y.as<T>());
+        gemm(td.as<int32_t>() + t0, tb.as<int64_t>() + t0, tn.as<int32_t>() + t0, nt, nullptr,
+             pair_src.as<int32_t>(), m2l_tab.as<T>(), M.as<T>(), Y.as<T>());
     }
 
     void l2l_products(int l) {  // L2L products Yo of the children on level l (l >= 3)
         const int64_t t0 = l2l_tiles[l], nt = l2l_tiles[l + 1] - l2l_tiles[l];
-        if (nt)
-            m2l_gemm_kernel<P, T><<<counted((unsigned)nt), 256, gemm_smem, stream>>>(
-                oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0, oct_tile_count.as<int32_t>() + t0,
-                oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(), m, l2l_tab.as<T>(), Lc.as<T>(), Yo.as<T>());
+        gemm(oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0, oct_tile_count.as<int32_t>() + t0, nt,
+             oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(), l2l_tab.as<T>(), Lc.as<T>(), Yo.as<T>());
     }
 
     void reduce_locals(int l, int with_l2l, int with_v, int accumulate, bool with_x = false) {
@@ -1385,8 +1426,21 @@ struct Evaluator final : EvaluatorBase {
     // column j the image of the unit real input e_j, the real plane over the imaginary
     // plane) as the real 2n x 2n block [[A_r, -A_i], [A_i, A_r]], column-major, in T,
     // scaled by `scale` (exact: a power of two)
+    // (f64 up to p = 8: A_r and A_i packed as the tensor path's fragments, gemm_f64.cuh)
+    static constexpr size_t kHhSet = kDmma<true> ? (size_t)GemmF64<P, true>::TABLE : (size_t)NE * NE;
     static void hh_block(const std::vector<double>& host, int sets, double scale, std::vector<T>& out, size_t at) {
         const int n = NC;
+        if constexpr (kDmma<true>) {
+            for_chunks((size_t)sets, stage_threads((size_t)sets * kHhSet / 32), [&](size_t, size_t d0, size_t d1) {
+                for (size_t d = d0; d < d1; ++d)
+                    for (int part = 0; part < 2; ++part) {
+                        const double* h = host.data() + d * 2 * n * n + (size_t)part * n;
+                        pack_f64_table<P>(out.data() + at + d * kHhSet, part, 2,
+                                          [&](int i, int j) { return scale * h[(size_t)j * 2 * n + i]; });
+                    }
+            });
+            return;
+        }
         for (int d = 0; d < sets; ++d) {
             const double* h = host.data() + (size_t)d * 2 * n * n;
             T* o = out.data() + at + (size_t)d * NE * NE;
@@ -1427,16 +1481,14 @@ struct Evaluator final : EvaluatorBase {
                                           (int)smem));
             CUDA_TRY(cudaFuncSetAttribute(hh_expand_kernel<P, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-            if (GemmShape<P, T, true>::SMEM > 48 * 1024)
-                CUDA_TRY(cudaFuncSetAttribute(m2l_gemm_kernel<P, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              GemmShape<P, T, true>::SMEM));
+            gemm_setup<true>();
             if constexpr (kHhTensor) hh_tc_tiles();
             hh.built = true;
         }
         if (k == hh.k) return;
         const auto t0 = std::chrono::steady_clock::now();
         for (int l = 0; l < NL; ++l) hh.lv.kl[l] = k * plan.side * std::ldexp(1.0, -(l + 1));
-        const size_t set = (size_t)NE * NE;
+        const size_t set = kHhSet;
         std::vector<T> m2l(kHhTensor ? 0 : (size_t)std::max(NL - 2, 1) * 316 * set), m2m((size_t)NL * 8 * set),
             l2l((size_t)NL * 8 * set);
         std::vector<double> host, hm, hl;
@@ -1558,7 +1610,7 @@ struct Evaluator final : EvaluatorBase {
         const int64_t ns = dp.nsrc;
         const int L = plan.nlevels - 1;
         const int mv = 2 * m;
-        const size_t set = (size_t)NE * NE;
+        const size_t set = kHhSet;
         T* hM = hh.M.as<T>();
         T* hL = hh.L.as<T>();
         if (ns > 0)
@@ -1572,15 +1624,12 @@ struct Evaluator final : EvaluatorBase {
         if (plan.nleaves())
             hh_expand_kernel<P, T, false><<<counted((unsigned)plan.nleaves()), 32, esmem, stream>>>(
                 dp, hh.lv, 0, (int64_t)plan.nleaves(), nullptr, m, spos.as<T4>(), hq.as<Cplx<T>>(), hM);
-        constexpr int gsm = GemmShape<P, T, true>::SMEM;
         for (int l = L - 1; l >= 0; --l) {
             const int64_t t0 = m2m_tiles[l], nt = m2m_tiles[l + 1] - m2m_tiles[l];
             const int64_t n = m2m_start[l + 1] - m2m_start[l];
-            if (nt)
-                m2l_gemm_kernel<P, T, true><<<counted((unsigned)nt), 256, gsm, stream>>>(
-                    oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0,
-                    oct_tile_count.as<int32_t>() + t0, oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(), m,
-                    hh.m2m.as<T>() + (size_t)l * 8 * set, hM, hh.Yo.as<T>());
+            gemm<true>(oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0,
+                       oct_tile_count.as<int32_t>() + t0, nt, oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(),
+                       hh.m2m.as<T>() + (size_t)l * 8 * set, hM, hh.Yo.as<T>());
             if (n)
                 m2m_reduce_kernel<P, T><<<counted((unsigned)n), round32(NC), 0, stream>>>(
                     dp, m2m_par.as<int32_t>() + m2m_start[l], n, mv, hh.Yo.as<T>(), hM);
@@ -1598,22 +1647,18 @@ struct Evaluator final : EvaluatorBase {
         } else {
             for (int l = 2; l <= L; ++l) {
                 const int64_t t0 = lvl_tiles[l], nt = lvl_tiles[l + 1] - lvl_tiles[l];
-                if (nt)
-                    m2l_gemm_kernel<P, T, true><<<counted((unsigned)nt), 256, gsm, stream>>>(
-                        ltile_d.as<int32_t>() + t0, ltile_begin.as<int64_t>() + t0, ltile_count.as<int32_t>() + t0,
-                        nullptr, pair_src.as<int32_t>(), m, hh.m2l.as<T>() + (size_t)(l - 2) * 316 * set, hM,
-                        hh.Y.as<T>());
+                gemm<true>(ltile_d.as<int32_t>() + t0, ltile_begin.as<int64_t>() + t0, ltile_count.as<int32_t>() + t0,
+                           nt, nullptr, pair_src.as<int32_t>(), hh.m2l.as<T>() + (size_t)(l - 2) * 316 * set, hM,
+                           hh.Y.as<T>());
             }
         }
         // downward: per level the L2L products, the locals (L2L + V in offset order), P2L
         for (int l = 2; l <= L; ++l) {
             if (l >= 3) {
                 const int64_t t0 = l2l_tiles[l], nt = l2l_tiles[l + 1] - l2l_tiles[l];
-                if (nt)
-                    m2l_gemm_kernel<P, T, true><<<counted((unsigned)nt), 256, gsm, stream>>>(
-                        oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0,
-                        oct_tile_count.as<int32_t>() + t0, oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(), m,
-                        hh.l2l.as<T>() + (size_t)l * 8 * set, hL, hh.Yo.as<T>());
+                gemm<true>(oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0,
+                           oct_tile_count.as<int32_t>() + t0, nt, oct_pair_e.as<int64_t>(),
+                           oct_pair_src.as<int32_t>(), hh.l2l.as<T>() + (size_t)l * 8 * set, hL, hh.Yo.as<T>());
             }
             const int64_t b0 = plan.level_start[l], b1 = plan.level_start[l + 1];
             if (b1 > b0) {

@@ -1,0 +1,353 @@
+// The f64 near field (P2P) and output pass: Laplace 1/(4 pi r) and Helmholtz e^{ikr}/(4 pi r),
+// potential and gradient.
+//
+// What bounds it: the FP64 pipe (64 lanes an SM).  A Laplace pair with its gradient takes 18
+// of its instructions: 3 differences, 3 for r2, 5 for 1/r, 7 for the sums.
+//
+// Work split.  An item is up to 32 targets of one leaf in ns slots (a power of two); its
+// K = 32 / ns lanes a target share the sources, so a leaf's remainder of 5 targets keeps
+// 40 lanes' worth of work on 32 lanes instead of 5 (leaves hold about 24 targets on average:
+// a lane a target left a quarter to a half of the lanes idle).  The near row's sources, taken
+// as one run over its leaves, go through shared memory in flushes of 64, mapped to the target
+// leaf's frame as y = fma(r, u, c) (the leaf itself unchanged); each flush's partial sums are
+// added to the lane's totals in flush order, and the K lanes of a target are added by a fixed
+// tree at the end.  With few items the flushes are dealt to W warps of a block and their
+// partials added in flush order all the same, so a target's sums are the same floats whatever
+// the number of items in the plan.
+//
+// The rules of the reference's device kernels hold: d = u_t - y, r2 by explicit fma, and a
+// pair is left out iff r2 == 0 (its 1/r is then 0).  The sum is added to the far-field partial
+// and scaled once, phi = phi_hat/(4 pi r_t), g = g_hat/((4 pi r_t) r_t)
+// (fmm-exec/src/fmm.rs:4750-4778), in caller order.
+#pragma once
+
+#include "helmholtz.cuh"
+#include "kernels.cuh"
+
+namespace fmmb {
+
+// 1 / sqrt(r2), 0 at r2 == 0.  The hardware's estimate of the high word has 21 significant
+// bits, so its square is exact and e = 1 - r2 y^2 takes one rounding; a third-order step
+// (Householder's, y (1 + e/2 + 3 e^2 / 8)) then leaves e^3 5/16 < 2^-57 beside the last
+// fma's rounding: 0.6 ulp measured against 0.5 for rsqrt(), at five instructions instead of
+// its slow-path tests.  Below 2^-1007 (and at 0) the library's form.
+__device__ __forceinline__ double inv_dist(double r2) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+    const double e = __fma_rn(-r2, y * y, 1.0);
+    double z = __fma_rn(y * e, __fma_rn(0.375, e, 0.5), y);
+    if (__double2hiint(r2) < 0x01000000) z = r2 == 0.0 ? 0.0 : rsqrt(r2);
+    return z;
+}
+
+// The Laplace pair of VB charge vectors (the geometry formed once).
+template <bool GRAD_, int VB_>
+struct NearLaplace {
+    static constexpr bool GRAD = GRAD_;
+    static constexpr int VB = VB_;
+    static constexpr int Q = VB;                       // doubles of a source's charges
+    static constexpr int C = VB * (GRAD ? 4 : 1);      // sums a target
+    struct Const {};
+    __device__ static __forceinline__ void pair(const Const&, double dx, double dy, double dz, const double* q,
+                                                double (&a)[C]) {
+        const double r2 = pair_r2<double>(dx, dy, dz);
+        const double y = inv_dist(r2);
+        const double y3 = GRAD ? y * (y * y) : 0.0;
+#pragma unroll
+        for (int b = 0; b < VB; ++b) {
+            double* s = a + b * (GRAD ? 4 : 1);
+            s[0] = __fma_rn(q[b], y, s[0]);
+            if (GRAD) {
+                const double w = -(q[b] * y3);
+                s[1] = __fma_rn(w, dx, s[1]);
+                s[2] = __fma_rn(w, dy, s[2]);
+                s[3] = __fma_rn(w, dz, s[3]);
+            }
+        }
+    }
+};
+
+// The Helmholtz pair (helmholtz.cuh's term): phi += q e / r, g += q ((damping - 1) + i phase)
+// e d / r^3, e = exp(damping) (cos phase + i sin phase); 1/r and its powers from one inverse
+// square root, r rounded from r2 / r with one correction step.
+template <bool GRAD_>
+struct NearHelmholtz {
+    static constexpr bool GRAD = GRAD_;
+    static constexpr int VB = 1;
+    static constexpr int Q = 2;
+    static constexpr int C = GRAD ? 8 : 2;
+    struct Const {
+        double kre, kim;
+    };
+    __device__ static __forceinline__ void pair(const Const& k, double dx, double dy, double dz, const double* q,
+                                                double (&a)[C]) {
+        const double r2 = pair_r2<double>(dx, dy, dz);
+        const double y = inv_dist(r2);
+        double r = r2 * y;
+        r = __fma_rn(0.5 * y, __fma_rn(-r, r, r2), r);
+        const double phase = k.kre * r;
+        double sn, cs;
+        sincos(phase, &sn, &cs);
+        double damping = 0.0;
+        if (k.kim != 0.0) {
+            damping = -(k.kim * r);
+            const double decay = exp(damping);
+            sn *= decay;
+            cs *= decay;
+        }
+        const double qr = q[0] * cs - q[1] * sn, qi = q[0] * sn + q[1] * cs;  // q e
+        a[0] = __fma_rn(qr, y, a[0]);
+        a[1] = __fma_rn(qi, y, a[1]);
+        if (GRAD) {
+            const double y3 = y * (y * y), f = damping - 1.0;
+            const double gr = (qr * f - qi * phase) * y3, gi = (qr * phase + qi * f) * y3;
+            a[2] = __fma_rn(gr, dx, a[2]);
+            a[3] = __fma_rn(gi, dx, a[3]);
+            a[4] = __fma_rn(gr, dy, a[4]);
+            a[5] = __fma_rn(gi, dy, a[5]);
+            a[6] = __fma_rn(gr, dz, a[6]);
+            a[7] = __fma_rn(gi, dz, a[7]);
+        }
+    }
+};
+
+// Where the sums go.  Laplace: mode 0 adds the far partial and writes the scaled output in
+// caller order, 1 adds into the leaf-order store (level calls), 2 writes the near field alone
+// in leaf order; far_phi [v][t], far_g [v][t][3].  Helmholtz: mode 0 with complex far partials
+// (null: none), [v][t][2] and [v][t][6].
+struct NearArgs {
+    DevPlan plan;
+    P2pItems items;
+    int m, near, mode;
+    const double4* spos;
+    const double* sq;  // [v][point] (Helmholtz: complex)
+    const double4* tpos;
+    double *far_phi, *far_g, *out_phi, *out_g;
+    double k_re, k_im;  // the physical wavenumber
+};
+
+constexpr int kNearFlush = 64;    // sources a flush
+constexpr int kNearRecs = 64;     // near entries held at once
+constexpr int kNearWarps = 4;     // warps (items) a block when items are not shared
+
+template <class PK>
+constexpr int near_stage_doubles() {  // x, y, z, charges, in 16-byte pairs
+    return (3 + PK::Q + 1) / 2 * 2;
+}
+
+// SHARE: the block's warps share one item (its flushes dealt round robin); else a warp an item.
+template <class PK, bool SHARE>
+__global__ void __launch_bounds__(SHARE ? 256 : 32 * kNearWarps) near_f64_kernel(NearArgs A) {
+    constexpr int SD = near_stage_doubles<PK>(), C = PK::C;
+    constexpr bool HELM = PK::Q == 2 && PK::C == (PK::GRAD ? 8 : 2) && PK::VB == 1;
+    constexpr int RW = SHARE ? 1 : kNearWarps;  // record sets a block
+    static_assert(C * 32 <= kNearFlush * SD, "a warp's partial sums fit its stage");
+    __shared__ double4 rec_frame[RW][kNearRecs];
+    __shared__ int64_t rec_s0[RW][kNearRecs];
+    __shared__ int rec_pre[RW][kNearRecs + 1];
+    extern __shared__ __align__(16) double near_stage[];  // [warps][SD / 2][flush][2]
+    const DevPlan& plan = A.plan;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int W = SHARE ? (int)(blockDim.x >> 5) : 1, ws = SHARE ? warp : 0, rw = SHARE ? 0 : warp;
+    const int64_t item = SHARE ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kNearWarps + warp;
+    if (item >= A.items.count) return;
+    double2* st = reinterpret_cast<double2*>(near_stage) + (size_t)warp * (SD / 2) * kNearFlush;
+    const int leaf = A.items.leaf[item];
+    const int box = plan.leaf_box[leaf];
+    const int nn = A.items.n[item], ni = nn & 255, ns = nn >> 8;  // targets, slots (a power of two)
+    const int ti = lane & (ns - 1), kk = lane / ns, K = 32 / ns;
+    const int64_t t = A.items.t0[item] + (ti < ni ? ti : 0);
+    const double4 tp = A.tpos[t];
+    const int64_t n0 = plan.near_row[leaf], n1 = A.near ? plan.near_row[leaf + 1] : n0;
+    const int64_t nt = plan.ntgt;
+    const double rt = (plan.box_side ? plan.box_side[box] : plan.side) * pow2d(-(plan.level[box] + 1));
+    const double phi_scale = 4.0 * 3.141592653589793 * rt;
+    const double g_scale = phi_scale * rt;
+    typename PK::Const kc;
+    if constexpr (HELM) {
+        kc.kre = A.k_re * rt;  // k_l = k r_l
+        kc.kim = A.k_im * rt;
+    }
+    for (int v0 = 0; v0 < A.m; v0 += PK::VB) {
+        const int nb = A.m - v0 < PK::VB ? A.m - v0 : PK::VB;
+        double acc[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) acc[c] = 0.0;
+        for (int64_t e0 = n0; e0 < n1; e0 += kNearRecs) {
+            // the records of up to 64 near entries: frame, first source, sources before it
+            const int ne = (int)(n1 - e0 < kNearRecs ? n1 - e0 : kNearRecs);
+            if (!SHARE || ws == 0) {
+                int cnt[2] = {0, 0};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int e = lane + 32 * h;
+                    if (e >= ne) continue;
+                    const int sl = plan.near_col[e0 + e];
+                    double c[3] = {0.0, 0.0, 0.0}, r = 1.0;  // the leaf itself: y = fma(1, u, 0) = u
+                    if (sl != leaf) rel_frame<double>(plan, plan.leaf_box[sl], box, c, r);
+                    rec_frame[rw][e] = make_double4(c[0], c[1], c[2], r);
+                    const int64_t s0 = plan.src_start[sl];
+                    rec_s0[rw][e] = s0;
+                    cnt[h] = (int)(plan.src_start[sl + 1] - s0);
+                }
+                int base = 0;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    int x = cnt[h];
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int y = __shfl_up_sync(0xffffffffu, x, o);
+                        if (lane >= o) x += y;
+                    }
+                    rec_pre[rw][lane + 32 * h] = base + x - cnt[h];
+                    base += __shfl_sync(0xffffffffu, x, 31);
+                }
+                if (lane == 0) rec_pre[rw][kNearRecs] = base;
+            }
+            if (SHARE)
+                __syncthreads();
+            else
+                __syncwarp();
+            const int tot = rec_pre[rw][kNearRecs];
+            const int nfl = (tot + kNearFlush - 1) / kNearFlush;
+            // a lane's two sources of flush f, mapped; past the end: no charge, away from any target
+            auto fetch = [&](int f, double (&s)[2][SD]) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int pos = f * kNearFlush + lane + 32 * h;
+#pragma unroll
+                    for (int c = 0; c < SD; ++c) s[h][c] = c < 3 ? 1024.0 : 0.0;
+                    if (pos >= tot) continue;
+                    int lo = 0;  // the last entry starting at or before pos
+#pragma unroll
+                    for (int b = kNearRecs / 2; b; b >>= 1)
+                        if (lo + b < ne && rec_pre[rw][lo + b] <= pos) lo += b;
+                    const double4 fr = rec_frame[rw][lo];
+                    const int64_t si = rec_s0[rw][lo] + (pos - rec_pre[rw][lo]);
+                    const double4 u = A.spos[si];
+                    s[h][0] = map_coord<double>(fr.w, u.x, fr.x);
+                    s[h][1] = map_coord<double>(fr.w, u.y, fr.y);
+                    s[h][2] = map_coord<double>(fr.w, u.z, fr.z);
+                    if constexpr (HELM) {
+                        const double2 q = reinterpret_cast<const double2*>(A.sq)[(int64_t)v0 * plan.nsrc + si];
+                        s[h][3] = q.x;
+                        s[h][4] = q.y;
+                    } else {
+#pragma unroll
+                        for (int b = 0; b < PK::VB; ++b)
+                            if (b < nb) s[h][3 + b] = A.sq[(int64_t)(v0 + b) * plan.nsrc + si];
+                    }
+                }
+            };
+            double nxt[2][SD];
+            if (ws < nfl) fetch(ws, nxt);
+            for (int f = ws; f - ws < nfl; f += W) {  // rounds of W flushes (every warp the same count)
+                const bool have = f < nfl;
+                double p[C];
+#pragma unroll
+                for (int c = 0; c < C; ++c) p[c] = 0.0;
+                if (have) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int c = 0; c < SD / 2; ++c)
+                            st[c * kNearFlush + lane + 32 * h] = make_double2(nxt[h][2 * c], nxt[h][2 * c + 1]);
+                    __syncwarp();
+                    if (f + W < nfl) fetch(f + W, nxt);  // in flight while this flush is summed
+                    const int cnt = tot - f * kNearFlush < kNearFlush ? tot - f * kNearFlush : kNearFlush;
+#pragma unroll 4
+                    for (int s = kk; s < (cnt + K - 1) / K * K; s += K) {
+                        double w[SD];
+#pragma unroll
+                        for (int c = 0; c < SD / 2; ++c) {
+                            const double2 x = st[c * kNearFlush + s];
+                            w[2 * c] = x.x;
+                            w[2 * c + 1] = x.y;
+                        }
+                        PK::pair(kc, sub_rn<double>(tp.x, w[0]), sub_rn<double>(tp.y, w[1]), sub_rn<double>(tp.z, w[2]),
+                                 w + 3, p);
+                    }
+                    __syncwarp();
+                }
+                if (SHARE) {
+                    // the round's partials added in flush order
+                    double* ps = reinterpret_cast<double*>(st);
+                    if (have)
+#pragma unroll
+                        for (int c = 0; c < C; ++c) ps[c * 32 + lane] = p[c];
+                    __syncthreads();
+                    if (ws == 0) {
+                        const int nw = nfl - f < W ? nfl - f : W;
+                        for (int w = 0; w < nw; ++w)
+#pragma unroll
+                            for (int c = 0; c < C; ++c)
+                                acc[c] += near_stage[(size_t)w * SD * kNearFlush + c * 32 + lane];
+                    }
+                    __syncthreads();
+                } else {
+#pragma unroll
+                    for (int c = 0; c < C; ++c) acc[c] += p[c];
+                }
+            }
+            if (SHARE)
+                __syncthreads();  // the records are read
+            else
+                __syncwarp();
+        }
+        if (SHARE && ws != 0) continue;
+        // the K lanes of a target
+        for (int o = ns; o < 32; o <<= 1)
+#pragma unroll
+            for (int c = 0; c < C; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+        if (kk != 0 || ti >= ni) continue;
+        if constexpr (HELM) {
+            const int64_t at = (int64_t)v0 * nt + t;
+            const int64_t i = (int64_t)v0 * nt + plan.tgt_perm[t];
+            if (A.far_phi) {  // the far field's partials, added after the near sums
+                acc[0] += A.far_phi[2 * at];
+                acc[1] += A.far_phi[2 * at + 1];
+                if (PK::GRAD)
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) acc[2 + c] += A.far_g[6 * at + c];
+            }
+            A.out_phi[2 * i] = acc[0] / phi_scale;
+            A.out_phi[2 * i + 1] = acc[1] / phi_scale;
+            if (PK::GRAD)
+#pragma unroll
+                for (int c = 0; c < 6; ++c) A.out_g[6 * i + c] = acc[2 + c] / g_scale;
+        } else {
+#pragma unroll
+            for (int b = 0; b < PK::VB; ++b) {
+                if (b >= nb) break;
+                const double* a = acc + b * (PK::GRAD ? 4 : 1);
+                const int64_t at = (int64_t)(v0 + b) * nt + t;
+                if (A.mode == 2) {
+                    A.out_phi[at] = a[0];
+                    if (PK::GRAD)
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) A.out_g[3 * at + k] = a[1 + k];
+                    continue;
+                }
+                const double ph = A.far_phi[at] + a[0];
+                if (A.mode == 1) {
+                    A.far_phi[at] = ph;
+                    if (PK::GRAD)
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) A.far_g[3 * at + k] += a[1 + k];
+                    continue;
+                }
+                const int64_t i = (int64_t)(v0 + b) * nt + plan.tgt_perm[t];
+                A.out_phi[i] = ph / phi_scale;
+                if (PK::GRAD)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) A.out_g[3 * i + k] = (A.far_g[3 * at + k] + a[1 + k]) / g_scale;
+            }
+        }
+    }
+}
+
+// launched from p2p_launch.cu (the kernels do not depend on the expansion order)
+void launch_near_laplace_f64(const NearArgs& a, bool gradients, cudaStream_t s);
+void launch_near_helmholtz_f64(const NearArgs& a, bool gradients, cudaStream_t s);
+
+}  // namespace fmmb
