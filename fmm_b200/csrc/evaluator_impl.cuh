@@ -22,6 +22,7 @@
 #include "kernels.cuh"
 #include "m2l_fused.cuh"
 #include "m2l_tc.cuh"
+#include "near_f64.cuh"
 #include "p2p_x2.cuh"
 
 namespace fmmb {
@@ -830,13 +831,16 @@ struct Evaluator final : EvaluatorBase {
         items.leaf = item_leaf.as<int32_t>();
         items.t0 = item_t0.as<int64_t>();
         items.count = (int64_t)il.size();
-        if constexpr (kMixed) build_p2p_lists();
+        build_p2p_lists();
     }
 
+    // The lists of a leaf's targets by item slots.  f64: one list in leaf order (its kernel
+    // takes each item's slots at run time), the same items.
     void build_p2p_lists() {
         std::vector<int32_t> lv[kP2pClasses], nv[kP2pClasses];
         std::vector<int64_t> tv[kP2pClasses];
         auto add = [&](int c, size_t j, int64_t t, int n) {
+            if (!kMixed) c = 0;
             lv[c].push_back((int32_t)j);
             tv[c].push_back(t);
             nv[c].push_back(n);
@@ -1401,19 +1405,17 @@ struct Evaluator final : EvaluatorBase {
             p2p_x2_shape<4>(range(2), near, accumulate, d_phi, fg, og, s);
             p2p_x2_shape<8>(range(3), near, accumulate, d_phi, fg, og, s);
         } else {
-            const int64_t i0 = item_lstart[l0], i1 = item_lstart[l1];
-            if (i1 <= i0) return;
-            P2pItems it{items.leaf + i0, items.t0 + i0, i1 - i0};
-            const unsigned g = (unsigned)((it.count + kP2pWarps - 1) / kP2pWarps);
-            if (gradients)
-                p2p_kernel<T, true><<<counted(g), 32 * kP2pWarps, 0, s>>>(
-                    dp, it, m, near, (T)kTheta2, spos.as<T4>(), sq.as<T>(), tpos.as<T4>(), close,
-                    far_phi.as<double>(), fg, accumulate, d_phi, og);
-            else
-                p2p_kernel<T, false><<<counted(g), 32 * kP2pWarps, 0, s>>>(
-                    dp, it, m, near, (T)kTheta2, spos.as<T4>(), sq.as<T>(), tpos.as<T4>(), close,
-                    far_phi.as<double>(), fg, accumulate, d_phi, og);
+            const P2pItems it = item_range(plist[0], plist_lstart[0][l0], plist_lstart[0][l1]);
+            if (!it.count) return;
+            counted(1);
+            launch_near_laplace_f64(near_args(it, near, accumulate, sq.as<double>(), far_phi.as<double>(), fg, d_phi, og),
+                                    gradients, s);
         }
+    }
+
+    NearArgs near_args(const P2pItems& it, int near, int mode, const double* q, double* fphi, double* fg, double* ophi,
+                       double* og, double kre = 0.0, double kim = 0.0) const {
+        return NearArgs{dp, it, m, near, mode, spos.as<double4>(), q, tpos.as<double4>(), fphi, fg, ophi, og, kre, kim};
     }
 
     // ---- the Helmholtz FMM (real k): complex expansions as row pairs, per-level tables ----
@@ -1727,15 +1729,23 @@ struct Evaluator final : EvaluatorBase {
                 return;
             }
         }
-        const unsigned g = (unsigned)((items.count + kHelmWarps - 1) / kHelmWarps);
-        if (gradients)
-            helm_p2p_kernel<T, true, kMixed><<<counted(g), 32 * kHelmWarps, 0, stream>>>(
-                dp, items, m, (T)kTheta2, kre, kim, spos.as<T4>(), hq.as<Cplx<T>>(), tpos.as<T4>(), close,
-                hq64.as<double2>(), far_phi, far_g, d_phi, d_grad);
-        else
-            helm_p2p_kernel<T, false, kMixed><<<counted(g), 32 * kHelmWarps, 0, stream>>>(
-                dp, items, m, (T)kTheta2, kre, kim, spos.as<T4>(), hq.as<Cplx<T>>(), tpos.as<T4>(), close,
-                hq64.as<double2>(), far_phi, nullptr, d_phi, nullptr);
+        if constexpr (kMixed) {
+            const unsigned g = (unsigned)((items.count + kHelmWarps - 1) / kHelmWarps);
+            if (gradients)
+                helm_p2p_kernel<T, true, kMixed><<<counted(g), 32 * kHelmWarps, 0, stream>>>(
+                    dp, items, m, (T)kTheta2, kre, kim, spos.as<T4>(), hq.as<Cplx<T>>(), tpos.as<T4>(), close,
+                    hq64.as<double2>(), far_phi, far_g, d_phi, d_grad);
+            else
+                helm_p2p_kernel<T, false, kMixed><<<counted(g), 32 * kHelmWarps, 0, stream>>>(
+                    dp, items, m, (T)kTheta2, kre, kim, spos.as<T4>(), hq.as<Cplx<T>>(), tpos.as<T4>(), close,
+                    hq64.as<double2>(), far_phi, nullptr, d_phi, nullptr);
+        } else {
+            counted(1);
+            launch_near_helmholtz_f64(near_args(plist[0], 1, 0, hq.as<double>(), const_cast<double*>(far_phi),
+                                                const_cast<double*>(far_g), d_phi, gradients ? d_grad : nullptr, kre,
+                                                kim),
+                                      gradients, stream);
+        }
     }
 
     // ---- the Helmholtz near field (all leaves' P2P level calls) ----

@@ -10,7 +10,7 @@
 // the level's wavenumber k_l = k r_0 2^-l (fmm-tables/src/helmholtz.rs:472), sources
 // mapped into the target leaf by y = fma(r, u, c); the output is phi / (4 pi r_t) and
 // grad / ((4 pi r_t) r_t) in caller order, as for Laplace.
-// Work split as p2p_kernel: one warp per item of up to 32 targets of one leaf, source
+// This kernel serves f32 (complex64; f64 runs near_f64.cuh): one warp per item of up to 32 targets of one leaf, source
 // leaves of the near row staged in shared memory, a partial per source leaf added into
 // f64 per-target sums.
 #pragma once

@@ -939,17 +939,10 @@ __device__ __forceinline__ void m2p_eval_mv(const float* M, int nb, float x, flo
 }
 
 // ---------------------------------------------------------------------------------
-// P2P + output pass.  One warp per work item = up to 32 targets of one leaf (lane =
-// target); the warp walks the leaf's near row (source leaves by leaf index) and stages
-// each source leaf's points in its own shared memory, mapped to the target leaf's
-// frame: y = fma(r, u_s, c) (CONVENTIONS 3.13 "Device kernels", rule 1), the leaf
-// itself unchanged.  Per pair d = u_t - y, r2 by explicit fma (rules 2-3), and the
-// pair is skipped by a select before rho meets a charge (rule 4): iff r2 == 0, the
-// coincidence rule of the reference.  This is the plain f64 kernel; the mixed form's
-// P2P is in p2p_x2.cuh (its near-singular pairs found by close_pairs_kernel below, whose
-// f32 r2 is formed with pair_r2).  The per-target sum is added to the far-field partial
-// and scaled once, phi = phi_hat/(4 pi r_t) and g = g_hat/((4 pi r_t) r_t)
-// (fmm-exec/src/fmm.rs:4750-4778), in caller order.
+// What the near-field kernels share (the f64 one is near_f64.cuh, the mixed one p2p_x2.cuh,
+// its near-singular pairs found by close_pairs_kernel below): a source point mapped to the
+// target leaf's frame, y = fma(r, u_s, c) (CONVENTIONS 3.13 "Device kernels", rule 1), the
+// pair's d = u_t - y and its r2 by explicit fma (rules 2-3), and the work items.
 // ---------------------------------------------------------------------------------
 constexpr int kP2pWarps = 4;
 constexpr int kP2pStage = 64;
@@ -1147,116 +1140,6 @@ static __global__ void close_map_kernel(DevPlan plan, ClosePairs close, double4*
         }
 }
 
-template <typename T, bool GRAD>
-__global__ void __launch_bounds__(128) p2p_kernel(DevPlan plan, P2pItems items, int m, int near, T theta2,
-                                                  const typename Vec4<T>::type* __restrict__ spos,
-                                                  const T* __restrict__ sq,
-                                                  const typename Vec4<T>::type* __restrict__ tpos, ClosePairs close,
-                                                  double* __restrict__ far_phi, double* __restrict__ far_g,
-                                                  int accumulate, double* __restrict__ out_phi,
-                                                  double* __restrict__ out_g) {
-    using T4 = typename Vec4<T>::type;
-    __shared__ T4 stage[kP2pWarps][kP2pStage];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t item = (int64_t)blockIdx.x * kP2pWarps + warp;
-    if (item >= items.count) return;
-    const int leaf = items.leaf[item];
-    const int box = plan.leaf_box[leaf];
-    const int64_t t1 = plan.tgt_start[leaf + 1];
-    const int64_t t = items.t0[item] + lane;
-    const bool valid = t < t1;
-    const int64_t n0 = plan.near_row[leaf], n1 = near ? plan.near_row[leaf + 1] : n0;
-    const int64_t nt = plan.ntgt;
-    T tx = T(0), ty = T(0), tz = T(0);
-    if (valid) {
-        T4 p4 = tpos[t];
-        tx = p4.x;
-        ty = p4.y;
-        tz = p4.z;
-    }
-    const double rt = (plan.box_side ? plan.box_side[box] : plan.side) * pow2d(-(plan.level[box] + 1));
-    const double phi_scale = 4.0 * 3.141592653589793 * rt;
-    const double g_scale = phi_scale * rt;
-    for (int v = 0; v < m; ++v) {
-        double aphi = 0.0, ag0 = 0.0, ag1 = 0.0, ag2 = 0.0;
-        for (int64_t e = n0; e < n1; ++e) {
-            const int sl = plan.near_col[e];
-            T c[3] = {T(0), T(0), T(0)}, r = T(1);
-            const bool self = sl == leaf;
-            if (!self) rel_frame<T>(plan, plan.leaf_box[sl], box, c, r);
-            const int64_t s0 = plan.src_start[sl], s1 = plan.src_start[sl + 1];
-            for (int64_t sb = s0; sb < s1; sb += kP2pStage) {
-                const int cnt = (int)((s1 - sb) < kP2pStage ? (s1 - sb) : kP2pStage);
-                for (int j = lane; j < cnt; j += 32) {
-                    T4 p4 = spos[sb + j];
-                    T4 y;
-                    y.x = self ? p4.x : map_coord<T>(r, p4.x, c[0]);
-                    y.y = self ? p4.y : map_coord<T>(r, p4.y, c[1]);
-                    y.z = self ? p4.z : map_coord<T>(r, p4.z, c[2]);
-                    y.w = sq[(int64_t)v * plan.nsrc + sb + j];
-                    stage[warp][j] = y;
-                }
-                __syncwarp();
-                T pphi = T(0), pg0 = T(0), pg1 = T(0), pg2 = T(0);
-#pragma unroll 4
-                for (int s = 0; s < cnt; ++s) {
-                    const T4 y = stage[warp][s];
-                    const T dx = sub_rn<T>(tx, y.x), dy = sub_rn<T>(ty, y.y), dz = sub_rn<T>(tz, y.z);
-                    const T r2 = pair_r2<T>(dx, dy, dz);
-                    const bool skip = r2 == T(0);
-                    const T rinv = skip ? T(0) : rsqrt(r2);
-                    const T qr = y.w * rinv;
-                    pphi += qr;
-                    if (GRAD) {
-                        const T qr3 = qr * rinv * rinv;
-                        pg0 -= qr3 * dx;
-                        pg1 -= qr3 * dy;
-                        pg2 -= qr3 * dz;
-                    }
-                }
-                aphi += (double)pphi;
-                if (GRAD) {
-                    ag0 += (double)pg0;
-                    ag1 += (double)pg1;
-                    ag2 += (double)pg2;
-                }
-                __syncwarp();
-            }
-        }
-        if (!valid) continue;
-        if (accumulate == 2) {  // near field alone, leaf order (added to the far field by output_kernel)
-            out_phi[(int64_t)v * nt + t] = aphi;
-            if (GRAD) {
-                double* o = out_g + ((int64_t)v * nt + t) * 3;
-                o[0] = ag0;
-                o[1] = ag1;
-                o[2] = ag2;
-            }
-            continue;
-        }
-        const double ph = far_phi[(int64_t)v * nt + t] + aphi;
-        if (accumulate) {  // level calls: add into the leaf-order store, scaled by output_kernel
-            far_phi[(int64_t)v * nt + t] = ph;
-            if (GRAD) {
-                double* fg = far_g + ((int64_t)v * nt + t) * 3;
-                fg[0] = fg[0] + ag0;
-                fg[1] = fg[1] + ag1;
-                fg[2] = fg[2] + ag2;
-            }
-            continue;
-        }
-        const int64_t i = plan.tgt_perm[t];
-        out_phi[(int64_t)v * nt + i] = ph / phi_scale;
-        if (GRAD) {
-            const double* fg = far_g + ((int64_t)v * nt + t) * 3;
-            double* o = out_g + ((int64_t)v * nt + i) * 3;
-            o[0] = (fg[0] + ag0) / g_scale;
-            o[1] = (fg[1] + ag1) / g_scale;
-            o[2] = (fg[2] + ag2) / g_scale;
-        }
-    }
-}
-
 // Output pass (fmm-kernels/src/movement.rs:411 gather_output with the scaling of
 // fmm-exec/src/fmm.rs:4750-4778): phi = phi_hat / (4 pi r_t) and
 // g = g_hat / ((4 pi r_t) r_t), leaf order -> caller order, phi_hat = far + near when the
@@ -1296,7 +1179,7 @@ static __global__ void output_kernel(DevPlan plan, int m, const double* __restri
         }
 }
 
-// Build time (mixed form): every near pair whose f32 r2, formed exactly as p2p_kernel
+// Build time (mixed form): every near pair whose f32 r2, formed exactly as the P2P kernel
 // forms it, is below theta2.  Appends (target, source point, source leaf); *count may
 // exceed cap, in which case the caller enlarges the buffer and runs it again.
 template <typename T>

@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(32 * W, 32 / W) p2p_x2_kernel(
         }
         if (valid) {
             if (near) close_sum_add<GRAD>(close, (int64_t)v * nt + t, aphi, ag0, ag1, ag2);
-            // both gradient sums hold -sum qr3 (t - y), as p2p_kernel's
+            // both gradient sums hold -sum qr3 (t - y), as the f64 near field's
             if (accumulate == 2) {  // near field alone, leaf order (added to the far field by output_kernel)
                 out_phi[(int64_t)v * nt + t] = aphi;
                 if (GRAD) {

@@ -1,0 +1,61 @@
+"""The f64 near field: items of every slot count (a leaf's remainders), flushes of exactly 64
+sources and one more, near rows of more entries than a warp has lanes, one to five
+charge vectors, coincident points, against direct sums; the complex (Helmholtz) form too."""
+import numpy as np
+import pytest
+
+import fmm_b200 as F
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(np.linalg.norm(np.asarray(a) - np.asarray(b)) / np.linalg.norm(np.asarray(b)))
+
+
+def direct(x, t, q, k=0.0):
+    d = t[:, None, :] - x[None, :, :]
+    r = np.sqrt((d * d).sum(-1))
+    with np.errstate(divide="ignore", invalid="ignore"):
+        inv = np.where(r > 0, 1.0 / r, 0.0)
+    g = np.exp(1j * k * r) * inv if k else inv
+    rad = g * (1j * k * r - 1.0) * inv * inv if k else -inv ** 3
+    f = 1.0 / (4.0 * np.pi)
+    return f * (g @ q).T, f * np.einsum("ij,ijk,jv->vik", rad, d, q)
+
+
+# a tree of one leaf: the evaluation is the near field alone.  1e-13: f64 sums of at most 200
+# terms that cancel (measured 1e-15)
+@pytest.mark.parametrize("m", [1, 2, 3, 5])
+def test_one_leaf_is_the_direct_sum(m):
+    rng = np.random.default_rng(m)
+    for nt in (1, 2, 4, 5, 8, 9, 16, 17, 24, 25, 32, 33, 57):
+        ns = int(rng.choice([1, 3, 31, 63, 64, 65, 128, 130]))
+        x, t = rng.random((ns, 3)), rng.random((nt, 3))
+        t[: min(nt, ns) // 2] = x[: min(nt, ns) // 2]  # coincident pairs are left out
+        q = rng.standard_normal((ns, m))
+        if ns == 1 and nt >= 1:
+            t[0] = t[0] + 0.25
+        fmm = F.FmmBuilder(3).gradients().vectors(m).max_points_per_leaf(200).build(x, t)
+        out = fmm.evaluate(q)
+        phi, g = direct(x, t, q)
+        assert rel(out.potential, phi) < 1e-13 and rel(out.gradient, g) < 1e-13, (ns, nt)
+        z = q + 1j * rng.standard_normal((ns, m))
+        hz = fmm.helmholtz_near(3.0, z)
+        phi, g = direct(x, t, z, 3.0)
+        assert rel(hz.potential, phi) < 1e-13 and rel(hz.gradient, g) < 1e-13, (ns, nt)
+        fmm.close()
+
+
+# 1e-12: the f64 path's bound against the oracle on the same tree and order
+def test_long_near_rows_match_oracle(oracle):
+    rng = np.random.default_rng(11)
+    x = np.concatenate([rng.random((300, 3)), 0.5 + 1e-3 * rng.random((6000, 3))])  # one dense corner
+    q = rng.standard_normal(len(x))
+    fmm = F.FmmBuilder(5).gradients().max_points_per_leaf(4).build(x)
+    arrays = fmm.plan_arrays()
+    assert np.diff(arrays["near_rows"]).max() > 32
+    out = fmm.evaluate(q)
+    phi, g = oracle.fmm(x, q, x, 5, 4, gradients=True, threads=8)
+    assert rel(out.potential, phi) < 1e-12 and rel(out.gradient, g) < 1e-12
+    fmm.close()
