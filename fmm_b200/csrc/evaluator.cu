@@ -440,7 +440,8 @@ void build_device(fmmgpu_fmm* f, const std::vector<double>& us, const std::vecto
         const size_t tsz = s.precision == FMMGPU_PRECISION_F64 ? 8 : 4;
         const size_t nsrc = P.src_perm.size(), ntgt = P.tgt_perm.size();
         const size_t y_vec = f->fused ? 0 : tsz * ys * (P.v.nnz() + 1);
-        const size_t per_vec = tsz * (2 * P.nboxes() * ms + P.nboxes() * ys + nsrc) + (tsz == 4 ? 8 * nsrc : 0) +
+        const size_t per_vec = tsz * ((P.x.nnz() ? 3 : 2) * P.nboxes() * ms + P.nboxes() * ys + nsrc) +
+                               (tsz == 4 ? 8 * nsrc : 0) +
                                8 * ntgt * (s.gradients ? 4 : 1) * 2 + 8 * ntgt * (s.gradients ? 4 : 1) + 8 * nsrc;
         size_t free_b = 0, total_b = 0;
         CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));

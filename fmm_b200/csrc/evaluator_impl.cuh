@@ -24,6 +24,7 @@
 #include "m2l_tc.cuh"
 #include "near_f64.cuh"
 #include "p2p_x2.cuh"
+#include "tree_chain.cuh"
 
 namespace fmmb {
 
@@ -33,7 +34,7 @@ static_assert(kX2Warps == 4, "EvaluatorBase::p2p_warps starts at the mixed P2P's
 // translation products, the per-level tables of one wavenumber, the far partials.
 struct HhState {
     double k = -1.0;  // the wavenumber of the tables held
-    DevBuf M, L, Y, Yo, m2l, m2m, l2l, far_phi, far_g;
+    DevBuf M, L, Lx, Y, Yo, m2l, m2m, l2l, far_phi, far_g;
     HhLevels lv{};
     bool built = false;
     // the mixed form's tensor-core M2L (p <= 10): tiles over every level, (level, offset,
@@ -68,6 +69,10 @@ struct Evaluator final : EvaluatorBase {
     // target) products, tiles of kGemmPairs; Yo holds one product row per child box
     DevBuf oct_tile_d, oct_tile_begin, oct_tile_count, oct_pair_e, oct_pair_src, Yo;
     std::vector<int64_t> m2m_tiles, l2l_tiles;  // tile ranges per level (nlevels + 1)
+    // the same pairs per level and octant (9 offsets a level) for the chains of small levels
+    // (tree_chain.cuh), the M2M parents' ranges on the device, and the pairs of each level
+    DevBuf up_off, down_off, m2m_start_d;
+    std::vector<int64_t> up_pairs, down_pairs;
     // M2L batches: pairs of all levels grouped by offset, in tiles
     DevBuf tile_d, tile_begin, tile_count, pair_e, pair_src, v_pos;
     int64_t ntiles = 0;
@@ -120,17 +125,15 @@ struct Evaluator final : EvaluatorBase {
     // target and vector (close_weights_kernel, close_sum_kernel)
     DevBuf close_w, close_acc, close_src32;
     // boxes with a nonempty X list, level by level (the P2L launches), the f32 P2L's
-    // per-entry records (XRec), and the X-list sums of the f32 P2L when it runs apart (Lx,
-    // a box's rows as in Lc): in the evaluation with the near-singular sums on near_stream,
-    // the P2L of every level runs there too, beside the upward pass, and the local reduce
-    // adds Lx last (the same floats as adding P2L into the stored locals)
+    // per-entry records (XRec), and the X-list sums (Lx, a box's rows as in Lc): the P2L of
+    // every level is one launch, beside the upward pass on near_stream unless kinds are
+    // timed, and the downward pass adds Lx last
     DevBuf xbox, xrec, Lx;
-    bool p2l_apart = false;  // set for one evaluation of that form
     std::vector<int64_t> xbox_start;
     // the near field summed apart on a second, lower-priority stream, joined by output_kernel
     DevBuf near_phi, near_g;
     cudaStream_t near_stream = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_x = nullptr, ev_join = nullptr;
     P2pItems items{};
     std::vector<int64_t> item_lstart;  // first work item of each level's leaves (nlevels + 1)
     std::vector<int32_t> item_leaf_h;  // the items' leaves (host copy, ascending)
@@ -278,8 +281,8 @@ struct Evaluator final : EvaluatorBase {
             }
             xbox_start[pl.nlevels] = (int64_t)xb.size();
             xbox.upload(xb);
-            if (kMixed && !xb.empty()) {  // the f32 P2L's entry records and its apart sums
-                Lx.alloc(sizeof(float) * (size_t)m * ms_of(P) * pl.nboxes());
+            if (!xb.empty()) Lx.alloc(sizeof(T) * (size_t)m * ms_of(P) * pl.nboxes());
+            if (kMixed && !xb.empty()) {  // the f32 P2L's entry records
                 xrec.alloc(sizeof(XRec) * (pl.x.nnz() + 1));
                 x_record_kernel<<<(unsigned)((xb.size() + 127) / 128), 128>>>(dp, xbox.as<int32_t>(),
                                                                               (int64_t)xb.size(), xrec.as<XRec>());
@@ -290,6 +293,7 @@ struct Evaluator final : EvaluatorBase {
         CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
         CUDA_TRY(cudaStreamCreateWithPriority(&near_stream, cudaStreamNonBlocking, least));
         CUDA_TRY(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+        CUDA_TRY(cudaEventCreateWithFlags(&ev_x, cudaEventDisableTiming));
         CUDA_TRY(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
         near_phi.alloc(sizeof(double) * (size_t)m * (dp.ntgt + 1));
         if (gradients) near_g.alloc(sizeof(double) * 3 * (size_t)m * (dp.ntgt + 1));
@@ -328,28 +332,96 @@ struct Evaluator final : EvaluatorBase {
     void gemm_setup() {
         if constexpr (kDmma<CPLX>) {
             using S = GemmF64<P, CPLX>;
-            CUDA_TRY(cudaFuncSetAttribute(gemm_f64_kernel<P, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            CUDA_TRY(cudaFuncSetAttribute(gemm_f64_kernel<P, CPLX, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          S::SMEM));
+            CUDA_TRY(cudaFuncSetAttribute(gemm_f64_kernel<P, CPLX, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           S::SMEM));
             int occ = 0;
-            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gemm_f64_kernel<P, CPLX>, 32 * S::WARPS,
-                                                                   S::SMEM));
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gemm_f64_kernel<P, CPLX, false>,
+                                                                   32 * S::WARPS, S::SMEM));
             gemm_blocks[CPLX] = std::max(1, occ * num_sms / S::SPLIT);
         } else if (GemmShape<P, T, CPLX>::SMEM > 48 * 1024) {
-            CUDA_TRY(cudaFuncSetAttribute(m2l_gemm_kernel<P, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          GemmShape<P, T, CPLX>::SMEM));
+            CUDA_TRY(cudaFuncSetAttribute(m2l_gemm_kernel<P, T, CPLX, false>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, GemmShape<P, T, CPLX>::SMEM));
+            CUDA_TRY(cudaFuncSetAttribute(m2l_gemm_kernel<P, T, CPLX, true>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, GemmShape<P, T, CPLX>::SMEM));
+        }
+        if constexpr (ChainShape<P, T, CPLX>::OK) {
+            CUDA_TRY(cudaFuncSetAttribute(chain_up_kernel<P, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          ChainShape<P, T, CPLX>::SMEM));
+            CUDA_TRY(cudaFuncSetAttribute(chain_down_kernel<P, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          ChainShape<P, T, CPLX>::SMEM));
         }
     }
-    template <bool CPLX = false>
+    // ADD: the products are added to the locals y (L2L), with the P2L sums lx when given
+    template <bool CPLX = false, bool ADD = false>
     void gemm(const int32_t* td, const int64_t* tb, const int32_t* tn, int64_t nt, const int64_t* pe,
-              const int32_t* ps, const T* tab, const T* x, T* y) {
+              const int32_t* ps, const T* tab, const T* x, T* y, const T* lx = nullptr) {
         if (nt <= 0) return;
         if constexpr (kDmma<CPLX>) {
             using S = GemmF64<P, CPLX>;
             const dim3 grid(counted((unsigned)std::min<int64_t>(nt, gemm_blocks[CPLX])), S::SPLIT);
-            gemm_f64_kernel<P, CPLX><<<grid, 32 * S::WARPS, S::SMEM, stream>>>(td, tb, tn, nt, pe, ps, m, tab, x, y);
+            gemm_f64_kernel<P, CPLX, ADD><<<grid, 32 * S::WARPS, S::SMEM, stream>>>(td, tb, tn, nt, pe, ps, m, tab, x,
+                                                                                    y, dp, lx);
         } else {
-            m2l_gemm_kernel<P, T, CPLX><<<counted((unsigned)nt), 256, GemmShape<P, T, CPLX>::SMEM, stream>>>(
-                td, tb, tn, pe, ps, m, tab, x, y);
+            // as many blocks a tile as leave the device about four blocks an SM, a vector each at least
+            const unsigned gy = (unsigned)std::min<int64_t>(m, std::max<int64_t>(1, 4 * num_sms / nt));
+            m2l_gemm_kernel<P, T, CPLX, ADD><<<dim3(counted((unsigned)nt), gy), 256, GemmShape<P, T, CPLX>::SMEM,
+                                               stream>>>(
+                td, tb, tn, pe, ps, m, tab, x, y, dp, lx);
+        }
+    }
+
+    template <bool CPLX, class F>
+    void timed(int kind, F&& f) {  // kinds are timed in the Laplace evaluation
+        if (CPLX)
+            f();
+        else
+            timer.run(kind, f);
+    }
+    // The M2M of every level, upward: runs of small levels as one chain launch each
+    // (tree_chain.cuh), the others by m2m_level.  tab: the octant tables, tab_level elements
+    // apart per level (0: one set); yo, mm: the products and the multipoles.
+    template <bool CPLX = false>
+    void upward(const T* tab, int64_t tab_level, T* yo, T* mm) {
+        for (int l = plan.nlevels - 2; l >= 0;) {
+            int l0 = l;  // the run l .. l0 + 1 of small levels
+            if constexpr (ChainShape<P, T, CPLX>::OK)
+                while (l0 >= 0 && up_pairs[l0] * m <= kChainRows) --l0;
+            if (l0 < l) {
+                if constexpr (ChainShape<P, T, CPLX>::OK)
+                    timed<CPLX>(kM2M, [&] {
+                        chain_up_kernel<P, T, CPLX><<<counted(8), kChainThreads, ChainShape<P, T, CPLX>::SMEM, stream>>>(
+                            dp, ChainPairs{up_off.as<int64_t>(), oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>()},
+                            m2m_par.as<int32_t>(), m2m_start_d.as<int64_t>(), l, l0 + 1, m, tab, tab_level, yo, mm);
+                    });
+                l = l0;
+            } else {
+                timed<CPLX>(kM2M, [&] { m2m_level<CPLX>(l, tab + l * tab_level, yo, mm); });
+                --l;
+            }
+        }
+    }
+    // The L2L of every level, downward, added to the V sums in ll, with the P2L sums lx.
+    template <bool CPLX = false>
+    void downward(const T* tab, int64_t tab_level, const T* lx, T* ll) {
+        const int L = plan.nlevels - 1;
+        for (int l = 3; l <= L;) {
+            int l1 = l;
+            if constexpr (ChainShape<P, T, CPLX>::OK)
+                while (l1 <= L && down_pairs[l1] * m <= kChainRows) ++l1;
+            if (l1 > l) {
+                if constexpr (ChainShape<P, T, CPLX>::OK)
+                    timed<CPLX>(kL2L, [&] {
+                        chain_down_kernel<P, T, CPLX><<<counted(8), kChainThreads, ChainShape<P, T, CPLX>::SMEM, stream>>>(
+                            dp, ChainPairs{down_off.as<int64_t>(), oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>()},
+                            l, l1 - 1, m, tab, tab_level, lx, ll);
+                    });
+                l = l1;
+            } else {
+                timed<CPLX>(kL2L, [&] { l2l_level<CPLX>(l, tab + l * tab_level, lx, ll); });
+                ++l;
+            }
         }
     }
 
@@ -359,6 +431,7 @@ struct Evaluator final : EvaluatorBase {
             cudaStreamDestroy(near_stream);
         }
         if (ev_fork) cudaEventDestroy(ev_fork);
+        if (ev_x) cudaEventDestroy(ev_x);
         if (ev_join) cudaEventDestroy(ev_join);
     }
 
@@ -489,30 +562,28 @@ struct Evaluator final : EvaluatorBase {
         gemm(ck_s_d.as<int32_t>() + c.s_t0, ck_s_begin.as<int64_t>() + c.s_t0, ck_s_count.as<int32_t>() + c.s_t0,
              c.s_nt, nullptr, ck_pair_src.as<int32_t>() + c.base, m2l_tab.as<T>(), M.as<T>(), Y.as<T>());
     }
-    void reduce_chunk(const Chunk& c, int with_l2l, int with_v, int accumulate) {
-        reduce_range(c.b0, c.b1, with_l2l, with_v, accumulate);
-    }
+    // the first box of a level that L2L reaches: the boxes before it take their P2L sums in
+    // the V reduce
+    int64_t first_l2l() const { return plan.level_start[std::min(3, plan.nlevels)]; }
 
-    // the local reduce of boxes [b0, b1): f32 a warp per box with 16-byte accesses, f64 a
-    // block per box (the same order of additions either way)
-    void reduce_range(int64_t b0, int64_t b1, int with_l2l, int with_v, int accumulate, bool with_x = false) {
+    // the V sums of boxes [b0, b1) (boxes before xend add their P2L sums): f32 a warp per box
+    // with 16-byte accesses, f64 a block per box (the same order of additions either way)
+    void reduce_range(int64_t b0, int64_t b1, int with_v, int accumulate, int64_t xend = 0) {
         if (b1 <= b0) return;
         if constexpr (kMixed) {
             const unsigned g = counted((unsigned)((b1 - b0 + 3) / 4));
-            const auto* yo = reinterpret_cast<const float*>(Yo.ptr);
             const auto* yv = reinterpret_cast<const float*>(Y.ptr);
             auto* lc = reinterpret_cast<float*>(Lc.ptr);
-            const auto* lx = with_x ? reinterpret_cast<const float*>(Lx.ptr) : nullptr;
+            const auto* lx = reinterpret_cast<const float*>(Lx.ptr);
             if (m == 1)
-                local_reduce4_kernel<P, true><<<g, 128, 0, stream>>>(dp, b0, b1, m, with_l2l, with_v, accumulate, yo,
-                                                                     yv, v_pos.as<int64_t>(), lc, lx);
+                local_reduce4_kernel<P, true><<<g, 128, 0, stream>>>(dp, b0, b1, m, with_v, accumulate, yv,
+                                                                     v_pos.as<int64_t>(), lc, lx, xend);
             else
-                local_reduce4_kernel<P, false><<<g, 128, 0, stream>>>(dp, b0, b1, m, with_l2l, with_v, accumulate,
-                                                                      yo, yv, v_pos.as<int64_t>(), lc, lx);
+                local_reduce4_kernel<P, false><<<g, 128, 0, stream>>>(dp, b0, b1, m, with_v, accumulate, yv,
+                                                                      v_pos.as<int64_t>(), lc, lx, xend);
         } else
             local_reduce_kernel<P, T><<<counted((unsigned)(b1 - b0)), round32(NC), 0, stream>>>(
-                dp, b0, b1, m, with_l2l, with_v, accumulate, Yo.as<T>(), Y.as<T>(), v_pos.as<int64_t>(),
-                Lc.as<T>());
+                dp, b0, b1, m, with_v, accumulate, Y.as<T>(), v_pos.as<int64_t>(), Lc.as<T>(), Lx.as<T>(), xend);
     }
 
     // The fused path's tiles (see m2l_fused.cuh).  A chunk closes once it holds about
@@ -736,19 +807,28 @@ struct Evaluator final : EvaluatorBase {
         std::vector<int64_t> tb, pe;
         m2m_tiles.assign(plan.nlevels + 1, 0);
         l2l_tiles.assign(plan.nlevels + 1, 0);
+        up_pairs.assign(plan.nlevels, 0);
+        down_pairs.assign(plan.nlevels, 0);
         auto octant = [&](int64_t c) {
             return (int)(((plan.idx[3 * c] & 1) << 2) | ((plan.idx[3 * c + 1] & 1) << 1) | (plan.idx[3 * c + 2] & 1));
         };
         for (int pass = 0; pass < 2; ++pass) {
             std::vector<int64_t>& ranges = pass == 0 ? m2m_tiles : l2l_tiles;
+            std::vector<int64_t>& pairs = pass == 0 ? up_pairs : down_pairs;
+            std::vector<int64_t> off((size_t)9 * plan.nlevels, 0);
             for (int l = 0; l < plan.nlevels; ++l) {
                 ranges[l] = (int64_t)td.size();
+                for (int o = 0; o < 9; ++o) off[9 * l + o] = (int64_t)pe.size();
                 const int cl = pass == 0 ? l + 1 : l;  // level of the children
                 if (cl >= plan.nlevels || (pass == 1 && l < 3)) continue;
                 std::vector<std::vector<int64_t>> by(8);
                 for (int64_t c = plan.level_start[cl]; c < plan.level_start[cl + 1]; ++c) {
                     if (pass == 0 ? plan.src_below[c] == 0 : plan.tgt_below[c] == 0) continue;
                     by[octant(c)].push_back(c);
+                }
+                for (int o = 0; o < 8; ++o) {
+                    pairs[l] += (int64_t)by[o].size();
+                    off[9 * l + o + 1] = off[9 * l + o] + (int64_t)by[o].size();
                 }
                 for (int o = 0; o < 8; ++o)
                     for (size_t s0 = 0; s0 < by[o].size(); s0 += kGemmPairs) {
@@ -764,7 +844,9 @@ struct Evaluator final : EvaluatorBase {
                     }
             }
             ranges[plan.nlevels] = (int64_t)td.size();
+            (pass == 0 ? up_off : down_off).upload(off);
         }
+        m2m_start_d.upload(m2m_start);
         oct_tile_d.upload(td);
         oct_tile_begin.upload(tb);
         oct_tile_count.upload(tc);
@@ -991,7 +1073,8 @@ struct Evaluator final : EvaluatorBase {
                                &near_phi, &near_g, &box_side, &v_pos, &xbox, &xrec, &Lx, &fu_tile_d, &fu_tile_begin,
                                &fu_tile_np, &fu_cta, &fu_pair_src, &fu_pair_tgt, &fu_img, &ck_tc_d, &ck_tc_begin,
                                &ck_tc_count, &ck_s_d, &ck_s_begin, &ck_s_count, &ck_pair_src, &st_rowpair,
-                               &st_xy, &st_zz, &st_idx, &close_w, &close_acc, &close_src32};
+                               &st_xy, &st_zz, &st_idx, &close_w, &close_acc, &close_src32, &up_off, &down_off,
+                               &m2m_start_d};
         size_t s = 0;
         for (auto* b : all) s += b->bytes;
         return s;
@@ -1014,31 +1097,25 @@ struct Evaluator final : EvaluatorBase {
             int64_t top = plan.nlevels > 2 ? plan.level_start[2] : (int64_t)plan.nboxes();
             CUDA_TRY(cudaMemsetAsync(Lc.ptr, 0, sizeof(T) * (size_t)m * ms_of(P) * top, stream));
         });
-        if (overlap && !timer.on && kinds == 3 && items.count) {
-            // the near field on near_stream (it needs only the charges) beside the far-field
-            // chain on the evaluator's stream; output_kernel adds them: far + near, the same
-            // addition as the fused P2P epilogue, so the same floats
+        // On near_stream beside the upward pass: every level's P2L (into Lx), then the
+        // near-singular sums, then with overlap the near field, summed apart (it needs only the
+        // charges) and added by output_kernel: far + near, the addition of the fused P2P
+        // epilogue, so the same floats.
+        const bool side = !timer.on;
+        const bool x = (kinds & 2) && Lx.ptr;
+        const bool apart = overlap && side && kinds == 3 && items.count;
+        const bool fork = side && (x || sums || apart);
+        if (fork) {
             CUDA_TRY(cudaEventRecord(ev_fork, stream));
             CUDA_TRY(cudaStreamWaitEvent(near_stream, ev_fork, 0));
-            close_sums(near_stream);
-            p2p_levels(0, plan.nlevels, 1, 2, near_phi.as<double>(), gradients ? near_g.as<double>() : nullptr,
-                       near_stream);
-            CUDA_TRY(cudaEventRecord(ev_join, near_stream));
-            run_far();
-            CUDA_TRY(cudaStreamWaitEvent(stream, ev_join, 0));
-            output(d_phi, d_grad, true);
-            CUDA_TRY(cudaGetLastError());
-            return;
-        }
-        const bool forked = sums && !timer.on;
-        // P2L apart on near_stream: the product path (all levels' M2L products at once)
-        p2l_apart = forked && (kinds & 2) && m2l_path == 1 && chunks.empty() && Lx.ptr;
-        if (forked) {
-            CUDA_TRY(cudaEventRecord(ev_fork, stream));
-            CUDA_TRY(cudaStreamWaitEvent(near_stream, ev_fork, 0));
-            if (p2l_apart)  // first: the first local reduce waits for it
-                for (int l = 2; l < plan.nlevels; ++l) p2l_level(l, true, near_stream);
-            close_sums(near_stream);
+            if (x) {  // first: the V reduce or the first L2L waits for it
+                p2l_rows(0, xbox_start[plan.nlevels], near_stream);
+                CUDA_TRY(cudaEventRecord(ev_x, near_stream));
+            }
+            if (sums) close_sums(near_stream);
+            if (apart)
+                p2p_levels(0, plan.nlevels, 1, 2, near_phi.as<double>(), gradients ? near_g.as<double>() : nullptr,
+                           near_stream);
             CUDA_TRY(cudaEventRecord(ev_join, near_stream));
         }
         if (!(kinds & 2)) {
@@ -1046,11 +1123,13 @@ struct Evaluator final : EvaluatorBase {
             CUDA_TRY(cudaMemsetAsync(far_phi.ptr, 0, far_phi.bytes, stream));
             CUDA_TRY(cudaMemsetAsync(far_g.ptr, 0, far_g.bytes, stream));
         } else {
-            run_far();
+            run_far(fork && x);
         }
-        if (forked && !p2l_apart) CUDA_TRY(cudaStreamWaitEvent(stream, ev_join, 0));
-        p2l_apart = false;
-        if (items.count) timer.run(kP2P, [&] { p2p_levels(0, plan.nlevels, kinds & 1, 0, d_phi, d_grad); });
+        if (fork) CUDA_TRY(cudaStreamWaitEvent(stream, ev_join, 0));
+        if (apart)
+            output(d_phi, d_grad, true);
+        else if (items.count)
+            timer.run(kP2P, [&] { p2p_levels(0, plan.nlevels, kinds & 1, 0, d_phi, d_grad); });
         CUDA_TRY(cudaGetLastError());
     }
 
@@ -1144,54 +1223,41 @@ struct Evaluator final : EvaluatorBase {
                 with_near && gradients ? near_g.as<double>() : nullptr, d_phi, gradients ? d_grad : nullptr);
     }
 
-    void run_far() {
-        const int L = plan.nlevels - 1;
+    // The far field into the leaves' partials.  x_side: the P2L sums come from near_stream
+    // (ev_x), else they are formed here.
+    void run_far(bool x_side) {
+        const int64_t nb = (int64_t)plan.nboxes(), b2 = plan.level_start[std::min(2, plan.nlevels)];
         // upward: P2M of every leaf, then M2M from level L-1 up to 0
         timer.run(kP2M, [&] { p2m_rows(0, (int64_t)plan.nleaves()); });
-        for (int l = L - 1; l >= 0; --l) timer.run(kM2M, [&] { m2m_level(l); });
+        upward(m2m_tab.as<T>(), 0, Yo.as<T>(), M.as<T>());
+        if (Lx.ptr && !x_side) timer.run(kP2L, [&] { p2l_rows(0, xbox_start[plan.nlevels], stream); });
+        // before the first read of the P2L sums
+        auto wait_x = [&] {
+            if (x_side) CUDA_TRY(cudaStreamWaitEvent(stream, ev_x, 0));
+        };
+        // the V sums of every level (all multipoles are final here): the products, then
+        // their sums; in chunks of boxes whose products fit the buffer; or fused
         if (m2l_path == 2) {
-            // downward, fused: per level the L2L part of the locals, then the V products
-            // added into them in row order, then P2L
-            for (int l = 2; l <= L; ++l) {
-                timer.run(kL2L, [&] {
-                    if (l >= 3) l2l_products(l);
-                    reduce_locals(l, l >= 3, 0, 0);
-                });
-                timer.run(kM2L, [&] { m2l_fused(l); });
-                timer.run(kP2L, [&] { p2l_level(l); });
-            }
-            timer.run(kFar, [&] { leaf_far(0, (int64_t)plan.nleaves(), 3); });
-            return;
-        }
-        if (!chunks.empty()) {
-            // downward, chunked: per level the L2L products, then chunk by chunk the M2L
-            // products and the locals (L2L + V in offset order), then P2L
-            for (int l = 2; l <= L; ++l) {
-                timer.run(kL2L, [&] {
-                    if (l >= 3) l2l_products(l);
-                });
-                for (const Chunk& c : chunks) {
-                    if (c.level != l) continue;
-                    timer.run(kM2L, [&] { m2l_chunk(c); });
-                    timer.run(kL2L, [&] { reduce_chunk(c, l >= 3, 1, 0); });
-                }
-                timer.run(kP2L, [&] { p2l_level(l); });
-            }
-            timer.run(kFar, [&] { leaf_far(0, (int64_t)plan.nleaves(), 3); });
-            return;
-        }
-        // M2L products of every level at once (all multipoles are final here)
-        timer.run(kM2L, [&] { m2l_products(-1); });
-        // P2L apart: its sums (on near_stream) are read by the first reduce
-        if (p2l_apart) CUDA_TRY(cudaStreamWaitEvent(stream, ev_join, 0));
-        // downward: for l = 2..L: L2L products, the local (L2L + V in offset order), then P2L
-        for (int l = 2; l <= L; ++l) {
-            timer.run(kL2L, [&] {
-                l2l_products(l);
-                reduce_locals(l, l >= 3, 1, 0, p2l_apart);
+            timer.run(kM2L, [&] {
+                CUDA_TRY(cudaMemsetAsync(Lc.ptr, 0, Lc.bytes, stream));
+                for (int l = 2; l < plan.nlevels; ++l) m2l_fused(l);
             });
-            if (!p2l_apart) timer.run(kP2L, [&] { p2l_level(l); });
+            wait_x();
+            timer.run(kL2L, [&] { reduce_range(b2, first_l2l(), 0, 1, first_l2l()); });
+        } else if (!chunks.empty()) {
+            wait_x();
+            for (const Chunk& c : chunks) {
+                if (c.level < 2) continue;
+                timer.run(kM2L, [&] { m2l_chunk(c); });
+                timer.run(kL2L, [&] { reduce_range(c.b0, c.b1, 1, 0, first_l2l()); });
+            }
+        } else {
+            timer.run(kM2L, [&] { m2l_products(-1); });
+            wait_x();
+            timer.run(kL2L, [&] { reduce_range(b2, nb, 1, 0, first_l2l()); });
         }
+        // downward: L = (L2L + V sum) + P2L sum, level by level
+        downward(l2l_tab.as<T>(), 0, Lx.as<T>(), Lc.as<T>());
         // leaves: L2P + M2P
         timer.run(kFar, [&] { leaf_far(0, (int64_t)plan.nleaves(), 3); });
     }
@@ -1221,14 +1287,24 @@ struct Evaluator final : EvaluatorBase {
                 dp, r0, r1, nullptr, m, spos.as<T4>(), sq.as<T>(), M.as<T>());
     }
 
-    void m2m_level(int l) {  // parents on level l from their children on level l + 1
+    template <bool CPLX = false>
+    void m2m_level(int l, const T* tab, T* yo, T* mm) {  // parents on level l from their children on level l + 1
         const int64_t t0 = m2m_tiles[l], nt = m2m_tiles[l + 1] - m2m_tiles[l];
         const int64_t n = m2m_start[l + 1] - m2m_start[l];
-        gemm(oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0, oct_tile_count.as<int32_t>() + t0, nt,
-             oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(), m2m_tab.as<T>(), M.as<T>(), Yo.as<T>());
+        gemm<CPLX>(oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0, oct_tile_count.as<int32_t>() + t0,
+                   nt, oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(), tab, mm, yo);
         if (n)
-            m2m_reduce_kernel<P, T><<<counted((unsigned)n), round32(NC), 0, stream>>>(
-                dp, m2m_par.as<int32_t>() + m2m_start[l], n, m, Yo.as<T>(), M.as<T>());
+            m2m_reduce_kernel<P, T><<<counted((unsigned)n), std::min(256, round32((CPLX ? 2 : 1) * m * NC)), 0, stream>>>(
+                dp, m2m_par.as<int32_t>() + m2m_start[l], n, CPLX ? 2 * m : m, yo, mm);
+    }
+
+    // L2L of the children on level l (l >= 3), added to their locals
+    template <bool CPLX = false>
+    void l2l_level(int l, const T* tab, const T* lx, T* ll) {
+        const int64_t t0 = l2l_tiles[l], nt = l2l_tiles[l + 1] - l2l_tiles[l];
+        gemm<CPLX, true>(oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0,
+                         oct_tile_count.as<int32_t>() + t0, nt, oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(),
+                         tab, ll, ll, lx);
     }
 
     // fused M2L of level l: L += the V products, in row order (after the L2L part)
@@ -1280,34 +1356,21 @@ struct Evaluator final : EvaluatorBase {
              pair_src.as<int32_t>(), m2l_tab.as<T>(), M.as<T>(), Y.as<T>());
     }
 
-    void l2l_products(int l) {  // L2L products Yo of the children on level l (l >= 3)
-        const int64_t t0 = l2l_tiles[l], nt = l2l_tiles[l + 1] - l2l_tiles[l];
-        gemm(oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0, oct_tile_count.as<int32_t>() + t0, nt,
-             oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(), l2l_tab.as<T>(), Lc.as<T>(), Yo.as<T>());
-    }
-
-    void reduce_locals(int l, int with_l2l, int with_v, int accumulate, bool with_x = false) {
-        reduce_range(plan.level_start[l], plan.level_start[l + 1], with_l2l, with_v, accumulate, with_x);
-    }
-
-    // P2L of the boxes of level l with an X list: added into the locals, or (apart, true)
-    // written into Lx on stream s for the local reduce to add (mixed form)
-    void p2l_level(int l, bool apart = false, cudaStream_t s = nullptr) {
-        const int64_t b0 = xbox_start[l], b1 = xbox_start[l + 1];
+    // P2L sums of the boxes [b0, b1) of the X box list into Lx, on stream s
+    void p2l_rows(int64_t b0, int64_t b1, cudaStream_t s) {
         if (b1 <= b0) return;
-        if (!s) s = stream;
-        float* out = reinterpret_cast<float*>(apart ? Lx.ptr : Lc.ptr);
+        auto* out = reinterpret_cast<float*>(Lx.ptr);
         if (kBflyP2L && m == 1)
             expand_bfly_kernel<P, true, false><<<counted((unsigned)(b1 - b0)), 32, 0, s>>>(
                 dp, b0, b1, xbox.as<int32_t>(), reinterpret_cast<const float4*>(spos.ptr), m,
-                reinterpret_cast<const float*>(sq.ptr), out, xrec.as<XRec>(), apart ? 1 : 0);
+                reinterpret_cast<const float*>(sq.ptr), out, xrec.as<XRec>());
         else if (kBflyP2L)
             expand_bfly_kernel<P, true, true><<<counted((unsigned)(b1 - b0)), 32, 0, s>>>(
                 dp, b0, b1, xbox.as<int32_t>(), reinterpret_cast<const float4*>(spos.ptr), m,
-                reinterpret_cast<const float*>(sq.ptr), out, xrec.as<XRec>(), apart ? 1 : 0);
-        else  // (f64: never apart)
+                reinterpret_cast<const float*>(sq.ptr), out, xrec.as<XRec>());
+        else
             expand_kernel<P, T, true><<<counted((unsigned)(b1 - b0)), 32, exp_smem(), s>>>(
-                dp, b0, b1, xbox.as<int32_t>(), m, spos.as<T4>(), sq.as<T>(), Lc.as<T>());
+                dp, b0, b1, xbox.as<int32_t>(), m, spos.as<T4>(), sq.as<T>(), Lx.as<T>());
     }
 
     void leaf_far(int64_t r0, int64_t r1, int mode) {  // L2P / M2P of leaves [r0, r1)
@@ -1469,6 +1532,8 @@ struct Evaluator final : EvaluatorBase {
             const size_t mv = 2 * (size_t)m;
             hh.M.alloc(sizeof(T) * mv * ms_of(P) * nb);
             hh.L.alloc(sizeof(T) * mv * ms_of(P) * nb);
+            CUDA_TRY(cudaMemset(hh.M.ptr, 0, hh.M.bytes));  // boxes without a source stay zero
+            if (xbox_start[plan.nlevels]) hh.Lx.alloc(sizeof(T) * mv * ms_of(P) * nb);
             hh.Y.alloc(sizeof(T) * mv * (kHhTensor ? 256 : ys_of(P)) * (plan.v.nnz() + 1));
             hh.Yo.alloc(sizeof(T) * mv * ys_of(P) * nb);
             hh.far_phi.alloc(sizeof(double) * 2 * (size_t)m * (dp.ntgt + 1));
@@ -1618,24 +1683,23 @@ struct Evaluator final : EvaluatorBase {
         if (ns > 0)
             helm_charge_kernel<T><<<counted((unsigned)((ns + 255) / 256)), 256, 0, stream>>>(
                 d_q, src_perm.as<int64_t>(), ns, m, qstride, hq.as<Cplx<T>>(), kMixed ? hq64.as<double2>() : nullptr);
-        CUDA_TRY(cudaMemsetAsync(hh.M.ptr, 0, hh.M.bytes, stream));
         const int64_t top = plan.nlevels > 2 ? plan.level_start[2] : (int64_t)plan.nboxes();
         CUDA_TRY(cudaMemsetAsync(hh.L.ptr, 0, sizeof(T) * (size_t)mv * ms_of(P) * top, stream));
         const size_t esmem = sizeof(double) * (2 * NC * 32 + 2 * (size_t)m * 32);
+        // beside the upward pass: the P2L of every level, into hh.Lx
+        const int64_t nx = xbox_start[plan.nlevels];
+        if (nx) {
+            CUDA_TRY(cudaEventRecord(ev_fork, stream));
+            CUDA_TRY(cudaStreamWaitEvent(near_stream, ev_fork, 0));
+            hh_expand_kernel<P, T, true><<<counted((unsigned)nx), 32, esmem, near_stream>>>(
+                dp, hh.lv, 0, nx, xbox.as<int32_t>(), m, spos.as<T4>(), hq.as<Cplx<T>>(), hh.Lx.as<T>());
+            CUDA_TRY(cudaEventRecord(ev_x, near_stream));
+        }
         // upward: P2M of every leaf, then M2M from level L-1 up to 0
         if (plan.nleaves())
             hh_expand_kernel<P, T, false><<<counted((unsigned)plan.nleaves()), 32, esmem, stream>>>(
                 dp, hh.lv, 0, (int64_t)plan.nleaves(), nullptr, m, spos.as<T4>(), hq.as<Cplx<T>>(), hM);
-        for (int l = L - 1; l >= 0; --l) {
-            const int64_t t0 = m2m_tiles[l], nt = m2m_tiles[l + 1] - m2m_tiles[l];
-            const int64_t n = m2m_start[l + 1] - m2m_start[l];
-            gemm<true>(oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0,
-                       oct_tile_count.as<int32_t>() + t0, nt, oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>(),
-                       hh.m2m.as<T>() + (size_t)l * 8 * set, hM, hh.Yo.as<T>());
-            if (n)
-                m2m_reduce_kernel<P, T><<<counted((unsigned)n), round32(NC), 0, stream>>>(
-                    dp, m2m_par.as<int32_t>() + m2m_start[l], n, mv, hh.Yo.as<T>(), hM);
-        }
+        upward<true>(hh.m2m.as<T>(), (int64_t)(8 * set), hh.Yo.as<T>(), hM);
         // M2L products of every level (their tables are per level): the mixed form on the
         // tensor cores in one launch over every level, f64 on the SIMT GEMM level by level
         if constexpr (kHhTensor) {
@@ -1654,34 +1718,23 @@ struct Evaluator final : EvaluatorBase {
                            hh.Y.as<T>());
             }
         }
-        // downward: per level the L2L products, the locals (L2L + V in offset order), P2L
-        for (int l = 2; l <= L; ++l) {
-            if (l >= 3) {
-                const int64_t t0 = l2l_tiles[l], nt = l2l_tiles[l + 1] - l2l_tiles[l];
-                gemm<true>(oct_tile_d.as<int32_t>() + t0, oct_tile_begin.as<int64_t>() + t0,
-                           oct_tile_count.as<int32_t>() + t0, nt, oct_pair_e.as<int64_t>(),
-                           oct_pair_src.as<int32_t>(), hh.l2l.as<T>() + (size_t)l * 8 * set, hL, hh.Yo.as<T>());
-            }
-            const int64_t b0 = plan.level_start[l], b1 = plan.level_start[l + 1];
-            if (b1 > b0) {
-                if constexpr (kHhTensor)
-                    hh_local_reduce_tc_kernel<P><<<counted((unsigned)(b1 - b0)), round32(NC), 0, stream>>>(
-                        dp, b0, b1, m, l >= 3, reinterpret_cast<const float*>(hh.Yo.ptr),
-                        reinterpret_cast<const float*>(hh.Y.ptr), v_pos.as<int64_t>(),
-                        reinterpret_cast<float*>(hh.L.ptr));
-                else if constexpr (kMixed)
-                    local_reduce4_kernel<P, false><<<counted((unsigned)((b1 - b0 + 3) / 4)), 128, 0, stream>>>(
-                        dp, b0, b1, mv, l >= 3, 1, 0, reinterpret_cast<const float*>(hh.Yo.ptr),
-                        reinterpret_cast<const float*>(hh.Y.ptr), v_pos.as<int64_t>(),
-                        reinterpret_cast<float*>(hh.L.ptr));
-                else
-                    local_reduce_kernel<P, T><<<counted((unsigned)(b1 - b0)), round32(NC), 0, stream>>>(
-                        dp, b0, b1, mv, l >= 3, 1, 0, hh.Yo.as<T>(), hh.Y.as<T>(), v_pos.as<int64_t>(), hL);
-            }
-            const int64_t x0 = xbox_start[l], x1 = xbox_start[l + 1];
-            if (x1 > x0)
-                hh_expand_kernel<P, T, true><<<counted((unsigned)(x1 - x0)), 32, esmem, stream>>>(
-                    dp, hh.lv, x0, x1, xbox.as<int32_t>(), m, spos.as<T4>(), hq.as<Cplx<T>>(), hL);
+        // the V sums of every level in one launch, then downward L = (L2L + V sum) + P2L sum
+        if (nx) CUDA_TRY(cudaStreamWaitEvent(stream, ev_x, 0));
+        const int64_t b2 = plan.level_start[std::min(2, plan.nlevels)], b1 = (int64_t)plan.nboxes();
+        if (b1 > b2) {
+            const T* lx = hh.Lx.as<T>();
+            if constexpr (kHhTensor)
+                hh_local_reduce_tc_kernel<P><<<counted((unsigned)(b1 - b2)), round32(NC), 0, stream>>>(
+                    dp, b2, b1, m, reinterpret_cast<const float*>(hh.Y.ptr), v_pos.as<int64_t>(),
+                    reinterpret_cast<float*>(hh.L.ptr), reinterpret_cast<const float*>(hh.Lx.ptr), first_l2l());
+            else if constexpr (kMixed)
+                local_reduce4_kernel<P, false><<<counted((unsigned)((b1 - b2 + 3) / 4)), 128, 0, stream>>>(
+                    dp, b2, b1, mv, 1, 0, reinterpret_cast<const float*>(hh.Y.ptr), v_pos.as<int64_t>(),
+                    reinterpret_cast<float*>(hh.L.ptr), reinterpret_cast<const float*>(hh.Lx.ptr), first_l2l());
+            else
+                local_reduce_kernel<P, T><<<counted((unsigned)(b1 - b2)), round32(NC), 0, stream>>>(
+                    dp, b2, b1, mv, 1, 0, hh.Y.as<T>(), v_pos.as<int64_t>(), hL, lx, first_l2l());
+            downward<true>(hh.l2l.as<T>(), (int64_t)(8 * set), lx, hL);
         }
         // leaves: L2P + M2P into the far partials, then the near field and the output pass
         if (plan.nleaves()) {
@@ -1777,36 +1830,49 @@ struct Evaluator final : EvaluatorBase {
     void op_level(int kind, int l) override {
         const int L = plan.nlevels - 1;
         const int64_t f0 = plan.leaf_level_start[l], f1 = plan.leaf_level_start[l + 1];
+        const int64_t b0 = plan.level_start[l], b1 = plan.level_start[l + 1];
         switch (kind) {
             case FMMGPU_OP_P2M: p2m_rows(f0, f1); break;
-            case FMMGPU_OP_M2M: if (l < L) m2m_level(l); break;
-            case FMMGPU_OP_L2L:
-                if (l >= 3) {
-                    l2l_products(l);
-                    reduce_locals(l, 1, 0, 1);
-                }
-                break;
+            case FMMGPU_OP_M2M: if (l < L) m2m_level(l, m2m_tab.as<T>(), Yo.as<T>(), M.as<T>()); break;
+            case FMMGPU_OP_L2L: if (l >= 3) l2l_level(l, l2l_tab.as<T>(), nullptr, Lc.as<T>()); break;
             case FMMGPU_OP_M2L:
-                if (l >= 2 && m2l_path == 2) {
+                if (l < 2) break;
+                if (m2l_path == 2) {
+                    // the fused products sum from zero, then the locals are added to them
+                    const size_t row = sizeof(T) * (size_t)m * ms_of(P), n = row * (size_t)(b1 - b0);
+                    T *lc = Lc.as<T>() + (size_t)b0 * m * ms_of(P), *yo = Yo.as<T>() + (size_t)b0 * m * ms_of(P);
+                    CUDA_TRY(cudaMemcpyAsync(yo, lc, n, cudaMemcpyDeviceToDevice, stream));
+                    CUDA_TRY(cudaMemsetAsync(lc, 0, n, stream));
                     m2l_fused(l);
-                } else if (l >= 2 && !chunks.empty()) {
+                    add_rows(yo, lc, (int64_t)(n / sizeof(T)));
+                } else if (!chunks.empty()) {
                     for (const Chunk& c : chunks)
                         if (c.level == l) {
                             m2l_chunk(c);
-                            reduce_chunk(c, 0, 1, 1);
+                            reduce_range(c.b0, c.b1, 1, 1);
                         }
-                } else if (l >= 2) {
+                } else {
                     m2l_products(l);
-                    reduce_locals(l, 0, 1, 1);
+                    reduce_range(b0, b1, 1, 1);
                 }
                 break;
-            case FMMGPU_OP_P2L: if (l >= 2) p2l_level(l); break;
+            case FMMGPU_OP_P2L:
+                if (l >= 2 && xbox_start[l + 1] > xbox_start[l]) {
+                    p2l_rows(xbox_start[l], xbox_start[l + 1], stream);
+                    reduce_range(b0, b1, 0, 1, b1);
+                }
+                break;
             case FMMGPU_OP_L2P: leaf_far(f0, f1, 5); break;
             case FMMGPU_OP_M2P: leaf_far(f0, f1, 6); break;
             case FMMGPU_OP_P2P: p2p_levels(l, l + 1, 1, 1, nullptr, nullptr); break;
             default: throw Failure(FMMGPU_INVALID_ARGUMENT, "unknown operator kind");
         }
         CUDA_TRY(cudaGetLastError());
+    }
+
+    // b[i] = a[i] + b[i]
+    void add_rows(const T* a, T* b, int64_t n) {
+        if (n > 0) add_rows_kernel<T><<<counted((unsigned)((n + 255) / 256)), 256, 0, stream>>>(n, a, b);
     }
 
     void op_output(double* d_phi, double* d_grad) override {

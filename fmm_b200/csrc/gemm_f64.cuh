@@ -30,7 +30,7 @@
 #include <cstdint>
 #include <vector>
 
-#include "harmonics.cuh"
+#include "kernels.cuh"
 
 namespace fmmb {
 
@@ -71,13 +71,20 @@ struct RowFrag {
     using S = GemmF64<P>;
     double a[S::KS8 > 0 ? S::KS8 : 1][4];
     double t0, t1;
-    // x0, x1: the lane's two rows (null: a row of zeros)
+    // x0, x1: the lane's two rows (null: a row of zeros); CG: past L1 (rows that another block
+    // of the launch wrote)
+    template <bool CG = false>
     __device__ __forceinline__ void load(const double* x0, const double* x1, int t) {
+        auto two = [](const double* x) {
+            const double2* p = reinterpret_cast<const double2*>(x);
+            return CG ? __ldcg(p) : *p;
+        };
+        auto one = [](const double* x) { return CG ? __ldcg(x) : *x; };
 #pragma unroll
         for (int k = 0; k < S::KS8; ++k) {
             double2 u = make_double2(0.0, 0.0), w = u;
-            if (x0) u = *reinterpret_cast<const double2*>(x0 + 8 * k + 2 * t);
-            if (x1) w = *reinterpret_cast<const double2*>(x1 + 8 * k + 2 * t);
+            if (x0) u = two(x0 + 8 * k + 2 * t);
+            if (x1) w = two(x1 + 8 * k + 2 * t);
             a[k][0] = u.x;
             a[k][1] = w.x;
             a[k][2] = u.y;
@@ -85,17 +92,9 @@ struct RowFrag {
         }
         t0 = t1 = 0.0;
         if (S::TAIL && 8 * S::KS8 + t < S::NC) {
-            if (x0) t0 = x0[8 * S::KS8 + t];
-            if (x1) t1 = x1[8 * S::KS8 + t];
+            if (x0) t0 = one(x0 + 8 * S::KS8 + t);
+            if (x1) t1 = one(x1 + 8 * S::KS8 + t);
         }
-    }
-    __device__ __forceinline__ void negate() {
-#pragma unroll
-        for (int k = 0; k < S::KS8; ++k)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) a[k][j] = -a[k][j];
-        t0 = -t0;
-        t1 = -t1;
     }
     // c += rows x the packed group at b (one table's KS8 steps and tail)
     __device__ __forceinline__ void mul(double (&c)[4], const double* b, int lane) const {
@@ -114,13 +113,17 @@ struct RowFrag {
 // pl): source row pair_src[p] * MV + MV/m v + pl of X, product row out * MV + MV/m v + pl of
 // Y with out = pair_e[p] when given, else p, MV = m (2 m complex).  Rows of X are ms_of(P)
 // doubles, of Y ys_of(P).
-template <int P, bool CPLX>
+// ADD: the L2L of a level, Y = the locals: the product is added to the child's row as
+// add_local does (its X sum from Lx).
+template <int P, bool CPLX, bool ADD>
 __global__ void __launch_bounds__(32 * GemmF64<P, CPLX>::WARPS, GemmF64<P, CPLX>::BLOCKS)
     gemm_f64_kernel(const int32_t* __restrict__ tile_d, const int64_t* __restrict__ tile_begin,
                     const int32_t* __restrict__ tile_count, int64_t ntiles, const int64_t* __restrict__ pair_e,
                     const int32_t* __restrict__ pair_src, int m, const double* __restrict__ tab,
-                    const double* __restrict__ X, double* __restrict__ Y) {
+                    const double* __restrict__ X, double* __restrict__ Y, DevPlan plan,
+                    const double* __restrict__ Lx) {
     using S = GemmF64<P, CPLX>;
+    static_assert(ms_of(P) == ys_of(P), "a local's row is laid out as a product's");
     constexpr int MS = ms_of(P), YS = ys_of(P), PT = S::PARTS;
     extern __shared__ __align__(16) double smem_tab[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -162,16 +165,19 @@ __global__ void __launch_bounds__(32 * GemmF64<P, CPLX>::WARPS, GemmF64<P, CPLX>
             RowFrag<P> xr, xi;
             const double *a0 = nullptr, *a1 = nullptr;
             int64_t o0 = 0, o1 = 0;
+            bool q0 = false, q1 = false;  // ADD: the rows' boxes take an X sum
             if (u < units) {
-                auto row = [&](int r, const double*& a, int64_t& o) {
+                auto row = [&](int r, const double*& a, int64_t& o, bool& q) {
                     if (r >= nrow) return;
                     const int pr = m == 1 ? r : r / m, v = m == 1 ? 0 : r % m;
                     const int64_t p = p0 + pr;
                     a = X + ((int64_t)pair_src[p] * m + v) * (PT * MS);
-                    o = ((pair_e ? pair_e[p] : p) * m + v) * (PT * YS);
+                    const int64_t b = pair_e ? pair_e[p] : p;
+                    o = (b * m + v) * (PT * YS);
+                    q = ADD && x_of(plan, b, Lx);
                 };
-                row(r0, a0, o0);
-                row(r1, a1, o1);
+                row(r0, a0, o0, q0);
+                row(r1, a1, o1, q1);
                 xr.load(a0, a1, t);
                 if (CPLX) xi.load(a0 ? a0 + MS : nullptr, a1 ? a1 + MS : nullptr, t);
             }
@@ -184,9 +190,14 @@ __global__ void __launch_bounds__(32 * GemmF64<P, CPLX>::WARPS, GemmF64<P, CPLX>
             auto store = [&](int n0, const double (&c)[4], int plane) {
                 const int n = n0 + 2 * t;
                 if (n >= S::NC) return;
-                // read once by the reduce: stream past L2
-                if (a0) __stcs(reinterpret_cast<double2*>(Y + o0 + plane * YS + n), make_double2(c[0], c[1]));
-                if (a1) __stcs(reinterpret_cast<double2*>(Y + o1 + plane * YS + n), make_double2(c[2], c[3]));
+                auto put = [&](int64_t at, bool q, double2 x) {
+                    if (ADD)
+                        add_local(Y + at, Lx + at, q, x);
+                    else  // read once by the reduce: stream past L2
+                        __stcs(reinterpret_cast<double2*>(Y + at), x);
+                };
+                if (a0) put(o0 + plane * YS + n, q0, make_double2(c[0], c[1]));
+                if (a1) put(o1 + plane * YS + n, q1, make_double2(c[2], c[3]));
             };
             if constexpr (!CPLX) {
                 int j = part;

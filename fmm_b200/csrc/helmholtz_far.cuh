@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(32) hh_expand_kernel(DevPlan plan, HhLevels lv
     const double kl = lv.kl[plan.level[box]], s = hh_scale(kl);
     const double pik = 4.0 * 3.14159265358979323846 * kl;
     T* outb = out + (int64_t)box * 2 * m * MS;
+    bool first = true;  // the row's sums start from its first 32 sources
     for (int e = 0; e < nent; ++e) {
         const int sleaf = SINGULAR ? plan.x_col[ent0 + e] : (int)row;
         double fc[3] = {0.0, 0.0, 0.0}, fr = 1.0;
@@ -366,10 +367,11 @@ __global__ void __launch_bounds__(32) hh_expand_kernel(DevPlan plan, HhLevels lv
                         }
                     }
                     T* o = outb + (int64_t)(2 * v) * MS + t;
-                    o[0] = (T)((double)o[0] + ar);
-                    o[MS] = (T)((double)o[MS] + ai);
+                    o[0] = first ? (T)ar : (T)((double)o[0] + ar);
+                    o[MS] = first ? (T)ai : (T)((double)o[MS] + ai);
                 }
             }
+            first = false;
             __syncwarp();
         }
     }
@@ -527,36 +529,50 @@ __global__ void __launch_bounds__(128) hh_leaf_far_kernel(DevPlan plan, HhLevels
     }
 }
 
-// The locals of one level from the tensor-core complex M2L's products (f32): for every box
+// The V sums from the tensor-core complex M2L's products (f32): for every box
 // with a target below it and every vector v,
-//   L_re = (L2L part) + sum_V (A_r x_re - A_i x_im),  L_im = (L2L part) + sum_V (A_i x_re + A_r x_im)
+//   L_re = sum_V (A_r x_re - A_i x_im),  L_im = sum_V (A_i x_re + A_r x_im)
 // with a pair's products Y[pos][2v + c][0..n) = A_r x_c and [128..128+n) = A_i x_c (row
-// stride 256), V entries in row order; the L2L part (with_l2l) from the SIMT complex GEMM's
-// rows 2v, 2v + 1 of stride ys_of(P).  Block per box, thread per slot.
+// stride 256), V entries in row order, four entries' loads in flight; boxes below xend add
+// their P2L sum.  Block per box, thread per slot.
 template <int P>
-__global__ void hh_local_reduce_tc_kernel(DevPlan plan, int64_t b0, int64_t b1, int m, int with_l2l,
-                                          const float* __restrict__ Yo, const float* __restrict__ Yv,
-                                          const int64_t* __restrict__ vpos, float* __restrict__ L) {
-    constexpr int NC = nc_of(P), YS = ys_of(P), MS = ms_of(P);
+__global__ void hh_local_reduce_tc_kernel(DevPlan plan, int64_t b0, int64_t b1, int m, const float* __restrict__ Yv,
+                                          const int64_t* __restrict__ vpos, float* __restrict__ L,
+                                          const float* __restrict__ Lx, int64_t xend) {
+    constexpr int NC = nc_of(P), MS = ms_of(P);
     const int64_t b = b0 + blockIdx.x;
     if (b >= b1 || plan.tgt_below[b] == 0) return;
     const int64_t e0 = plan.v_row[b], e1 = plan.v_row[b + 1];
     for (int v = 0; v < m; ++v)
         for (int t = threadIdx.x; t < NC; t += blockDim.x) {
             float sr = 0.0f, si = 0.0f;
-            if (with_l2l) {
-                sr = Yo[((int64_t)b * 2 * m + 2 * v) * YS + t];
-                si = Yo[((int64_t)b * 2 * m + 2 * v + 1) * YS + t];
+            int64_t e = e0;
+            for (; e + 4 <= e1; e += 4) {
+                float y[4][4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) y[j][c] = __ldcs(Yv + (vpos[e + j] * 2 * m + 2 * v) * 256 + 128 * c + t);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    sr += y[j][0] - y[j][3];
+                    si += y[j][1] + y[j][2];
+                }
             }
-            for (int64_t e = e0; e < e1; ++e) {
+            for (; e < e1; ++e) {
                 const float* y = Yv + (vpos[e] * 2 * m + 2 * v) * 256;
                 const float rr = __ldcs(y + t), ir = __ldcs(y + 128 + t);        // A_r x_re, A_i x_re
                 const float ri = __ldcs(y + 256 + t), ii = __ldcs(y + 384 + t);  // A_r x_im, A_i x_im
                 sr += rr - ii;
                 si += ir + ri;
             }
-            L[((int64_t)b * 2 * m + 2 * v) * MS + t] = sr;
-            L[((int64_t)b * 2 * m + 2 * v + 1) * MS + t] = si;
+            const int64_t at = ((int64_t)b * 2 * m + 2 * v) * MS + t;
+            if (has_x(plan, b, Lx, xend)) {
+                sr += Lx[at];
+                si += Lx[at + MS];
+            }
+            L[at] = sr;
+            L[at + MS] = si;
         }
 }
 

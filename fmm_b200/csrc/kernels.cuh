@@ -99,7 +99,9 @@ __global__ void charge_load_kernel(const double* __restrict__ q_caller, const in
 // sources = X-list leaves, frame (c(t|s), r(t|s))): one warp per row.  Each lane forms
 // the harmonics of one source and writes conj(X) into shared memory; lanes then sum
 // the 32 sources of a chunk per coefficient in source order.
-//   multipole: M_n^m += q conj R_n^m(u);  local: L_n^m += q conj I_n^m((u - c)/r)
+//   multipole: M_n^m = sum q conj R_n^m(u);  X sum: X_n^m = sum q conj I_n^m((u - c)/r)
+// P2L writes its sums to an array of their own (Lx, a box's rows as in Lc), so that every
+// level's P2L is one launch beside the upward pass; the downward pass adds them.
 // ---------------------------------------------------------------------------------
 template <int P, typename T, bool IRREG>
 __global__ void __launch_bounds__(32) expand_kernel(DevPlan plan, int64_t row_begin, int64_t row_end,
@@ -192,7 +194,7 @@ __global__ void __launch_bounds__(32) expand_kernel(DevPlan plan, int64_t row_be
                     T acc = T(0);
                     for (int j = 0; j < cnt; ++j) acc += Q[v * 32 + j] * S[c * 32 + j];
                     T* o = outb + (int64_t)v * ms_of(P) + c;
-                    if (first && !IRREG) *o = acc;
+                    if (first) *o = acc;
                     else *o += acc;
                 }
             first = false;
@@ -242,7 +244,7 @@ __global__ void __launch_bounds__(32) expand_bfly_kernel(DevPlan plan, int64_t r
                                                          const int32_t* __restrict__ rows,
                                                          const float4* __restrict__ spos, int m,
                                                          const float* __restrict__ sq, float* __restrict__ out,
-                                                         const XRec* __restrict__ xrec = nullptr, int overwrite = 0) {
+                                                         const XRec* __restrict__ xrec = nullptr) {
     constexpr int NC = nc_of(P);
     constexpr int NCP = ((NC + 31) / 32) * 32;
     const int lane = threadIdx.x;
@@ -362,22 +364,27 @@ __global__ void __launch_bounds__(32) expand_bfly_kernel(DevPlan plan, int64_t r
 #pragma unroll
     for (int i = 0; i < NCP / 32; ++i) {
         const int c = base + i;
-        if (c < NC) {
-            if (IRREG && !overwrite) o[c] += w[i];
-            else o[c] = w[i];
-        }
+        if (c < NC) o[c] = w[i];
     }
     }
 }
 
 // ---------------------------------------------------------------------------------
-// M2M and L2L run as batched GEMMs too (m2l_gemm_kernel with the 8 octant tables): the
-// product for child c is written to row c of Yo (M2M: T_o M_c; L2L: T_o L_parent(c)).
-// The reduces below then add rows in the reference's order.
+// M2M and L2L run as batched GEMMs too (the 8 octant tables): M2M's product T_o M_c is
+// written to row c of Yo and the reduce below adds a parent's children in the reference's
+// order; L2L's product T_o L_parent(c) is added to the child's local (add_local).
 // ---------------------------------------------------------------------------------
 
+// b += a (the fused M2L's level call: its sums start from zero, the locals are added to them)
+template <typename T>
+__global__ void add_rows_kernel(int64_t n, const T* __restrict__ a, T* __restrict__ b) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) b[i] = a[i] + b[i];
+}
+
 // M2M reduce for the parents of one level: M_p = sum over octants o (in order) of the
-// products of its children that hold a source.  Block per parent, thread per slot.
+// products of its children that hold a source.  Block per parent, its threads over the slots
+// of all vectors (a block of one vector's slots took 25 us a level with 16 vectors).
 template <int P, typename T>
 __global__ void m2m_reduce_kernel(DevPlan plan, const int32_t* __restrict__ parents, int64_t n, int m,
                                   const T* __restrict__ Yo, T* __restrict__ M) {
@@ -386,59 +393,89 @@ __global__ void m2m_reduce_kernel(DevPlan plan, const int32_t* __restrict__ pare
     if (j >= n) return;
     const int p = parents[j];
     const int c0 = plan.child_first[p];
-    for (int v = 0; v < m; ++v)
-        for (int i = threadIdx.x; i < NC; i += blockDim.x) {
-            T s = T(0);
+    for (int vi = threadIdx.x; vi < m * NC; vi += blockDim.x) {
+        const int v = vi / NC, i = vi % NC;
+        T s = T(0);
 #pragma unroll
-            for (int o = 0; o < 8; ++o)
-                if (plan.src_below[c0 + o]) s += Yo[((int64_t)(c0 + o) * m + v) * YS + i];
-            M[((int64_t)p * m + v) * ms_of(P) + i] = s;
-        }
+        for (int o = 0; o < 8; ++o)
+            if (plan.src_below[c0 + o]) s += Yo[((int64_t)(c0 + o) * m + v) * YS + i];
+        M[((int64_t)p * m + v) * ms_of(P) + i] = s;
+    }
 }
 
-// The locals of one level (>= 2), for every box with a target below it:
-//   L = (l >= 3 ? T_o L_parent : 0) + the V row's products in offset-index order
-// (the product of V entry e sits at row vpos[e] of Yv, its place in the M2L tile list),
-// written once (fmm-plan/src/operator.rs:34-45: L2L, then V by offset; X is added after).
-// Block per box, thread per slot; the V loop issues eight (then four) loads before adding them in order.
-// The evaluation writes L = Yo + sum_V Y (accumulate = 0); the level calls add into L:
-// L2L with with_v = 0, then M2L with with_l2l = 0, which gives the same floats when the
-// L2L call comes first (L starts at zero, so 0 + Yo = Yo).
+// A child's local in the downward pass: L = (T_o L_parent + S) + X, S its V sum (in L), X its
+// P2L sum when its X list is not empty (fmm-plan/src/operator.rs:34-45: the three are added,
+// here as whole sums).
+// x: whether the box takes an X sum (x_of, once a row).
+template <typename T>
+__device__ __forceinline__ bool x_of(const DevPlan& plan, int64_t box, const T* Lx) {
+    return Lx && plan.x_row[box + 1] > plan.x_row[box];
+}
+template <typename T>
+__device__ __forceinline__ void add_local(T* L, const T* Lx, bool x, T v) {
+    T s = v + __ldcg(L);
+    if (x) s += *Lx;
+    *L = s;
+}
+__device__ __forceinline__ void add_local(double* L, const double* Lx, bool x, double2 v) {
+    const double2 u = __ldcg(reinterpret_cast<const double2*>(L));
+    v.x += u.x;
+    v.y += u.y;
+    if (x) {
+        v.x += Lx[0];
+        v.y += Lx[1];
+    }
+    *reinterpret_cast<double2*>(L) = v;
+}
+
+// The V sums of boxes [b0, b1) with a target below them: S = the V row's products in
+// offset-index order (the product of V entry e sits at row vpos[e] of Yv, its place in the
+// M2L tile list), from zero.  The evaluation writes L = S for every level in one launch, since
+// no V sum waits for a parent's local, and the L2L pass adds its products to them; the level
+// calls add S into L (accumulate).  Boxes below xend add their P2L sum last: level 2's, which
+// no L2L reaches, or the boxes of a P2L level call (with_v = 0).
+// Block per box, thread per slot; sixteen loads in flight, added in order.
+template <typename T>
+__device__ __forceinline__ bool has_x(const DevPlan& plan, int64_t b, const T* Lx, int64_t xend) {
+    return Lx && b < xend && plan.x_row[b + 1] > plan.x_row[b];
+}
 template <int P, typename T>
-__global__ void local_reduce_kernel(DevPlan plan, int64_t b0, int64_t b1, int m, int with_l2l, int with_v,
-                                    int accumulate, const T* __restrict__ Yo, const T* __restrict__ Yv,
-                                    const int64_t* __restrict__ vpos, T* __restrict__ Lc) {
+__global__ void local_reduce_kernel(DevPlan plan, int64_t b0, int64_t b1, int m, int with_v, int accumulate,
+                                    const T* __restrict__ Yv, const int64_t* __restrict__ vpos, T* __restrict__ Lc,
+                                    const T* __restrict__ Lx, int64_t xend) {
     constexpr int NC = nc_of(P), YS = ys_of(P);
     const int64_t b = b0 + blockIdx.x;
     if (b >= b1 || plan.tgt_below[b] == 0) return;
     const int64_t e0 = plan.v_row[b], e1 = with_v ? plan.v_row[b + 1] : e0;
+    const bool with_x = has_x(plan, b, Lx, xend);
     for (int v = 0; v < m; ++v)
         for (int i = threadIdx.x; i < NC; i += blockDim.x) {
-            T s = accumulate ? Lc[(b * m + v) * ms_of(P) + i] : T(0);
-            if (with_l2l) s = accumulate ? s + Yo[(b * m + v) * YS + i] : Yo[(b * m + v) * YS + i];
+            T s = T(0);
             int64_t e = e0;
-            for (; e + 8 <= e1; e += 8) {  // eight rows in flight, added in row order
-                T y[8];
+            for (; e + 16 <= e1; e += 16) {  // sixteen rows in flight, added in row order
+                T y[16];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) y[j] = __ldcs(Yv + (vpos[e + j] * m + v) * YS + i);
+                for (int j = 0; j < 16; ++j) y[j] = __ldcs(Yv + (vpos[e + j] * m + v) * YS + i);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) s += y[j];
+                for (int j = 0; j < 16; ++j) s += y[j];
             }
             for (; e + 4 <= e1; e += 4) {
-                const T y0 = __ldcs(Yv + (vpos[e] * m + v) * YS + i), y1 = __ldcs(Yv + (vpos[e + 1] * m + v) * YS + i);
-                const T y2 = __ldcs(Yv + (vpos[e + 2] * m + v) * YS + i), y3 = __ldcs(Yv + (vpos[e + 3] * m + v) * YS + i);
-                s += y0;
-                s += y1;
-                s += y2;
-                s += y3;
+                T y[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) y[j] = __ldcs(Yv + (vpos[e + j] * m + v) * YS + i);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s += y[j];
             }
             for (; e < e1; ++e) s += __ldcs(Yv + (vpos[e] * m + v) * YS + i);
-            Lc[(b * m + v) * ms_of(P) + i] = s;
+            const int64_t at = (b * m + v) * ms_of(P) + i;
+            if (accumulate) s = Lc[at] + s;
+            if (with_x) s += Lx[at];
+            Lc[at] = s;
         }
 }
 
 // The same reduce for f32 expansions with 16-byte accesses: a warp per box (4 a block).
-// A box's m rows (its m vectors) are m NQ consecutive quads in the locals, in Yo and in
+// A box's m rows (its m vectors) are m NQ consecutive quads in the locals and in
 // each of its V entries' products (ys_of = ms_of = 4 NQ), so the lanes take quads f, f + 32,
 // ... of that run: every lane busy for any m (m = 16 at p = 6: 208 quads, 7 passes), 13 of
 // 32 when the lanes held one vector's quads.  Every coefficient adds the same terms in the
@@ -453,11 +490,10 @@ __device__ __forceinline__ void add4(float4& s, const float4 y) {
 }
 
 template <int P, bool ONE>  // ONE: m = 1 at compile time
-__global__ void __launch_bounds__(128, 4) local_reduce4_kernel(DevPlan plan, int64_t b0, int64_t b1, int m_,
-                                                            int with_l2l, int with_v, int accumulate,
-                                                            const float* __restrict__ Yo, const float* __restrict__ Yv,
+__global__ void __launch_bounds__(128, 4) local_reduce4_kernel(DevPlan plan, int64_t b0, int64_t b1, int m_, int with_v,
+                                                            int accumulate, const float* __restrict__ Yv,
                                                             const int64_t* __restrict__ vpos, float* __restrict__ Lc,
-                                                            const float* __restrict__ Lx = nullptr) {
+                                                            const float* __restrict__ Lx, int64_t xend) {
     constexpr int NC = nc_of(P), YS = ys_of(P), MS = ms_of(P), NQ = (NC + 3) / 4;
     static_assert(YS == MS && MS == 4 * NQ, "a box's m rows are m NQ consecutive quads");
     const int m = ONE ? 1 : m_;
@@ -465,20 +501,11 @@ __global__ void __launch_bounds__(128, 4) local_reduce4_kernel(DevPlan plan, int
     if (b >= b1 || plan.tgt_below[b] == 0) return;
     const int64_t e0 = plan.v_row[b], e1 = with_v ? plan.v_row[b + 1] : e0;
     const int F = m * NQ;  // the box's quads, all vectors
-    // P2L computed apart (Lx, the box's X-list sum, written by the P2L kernel beside the
-    // upward pass): added last, as the P2L kernel adds it to the stored locals otherwise
-    const bool with_x = Lx && plan.x_row[b + 1] > plan.x_row[b];
+    const bool with_x = has_x(plan, b, Lx, xend);
     for (int f = threadIdx.x & 31; f < F; f += 32) {
         const int q = f % NQ;  // the quad within its vector's row
         float4* out = reinterpret_cast<float4*>(Lc + b * m * MS) + f;
-        float4 s = accumulate ? *out : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (with_l2l) {
-            const float4 y = reinterpret_cast<const float4*>(Yo + b * m * YS)[f];
-            if (accumulate)
-                add4(s, y);
-            else
-                s = y;
-        }
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
         auto row = [&](int64_t e) { return __ldcs(reinterpret_cast<const float4*>(Yv + vpos[e] * m * YS) + f); };
         int64_t e = e0;
         for (; e + 16 <= e1; e += 16) {  // sixteen rows in flight, added in row order
@@ -503,6 +530,11 @@ __global__ void __launch_bounds__(128, 4) local_reduce4_kernel(DevPlan plan, int
             for (int j = 0; j < 4; ++j) add4(s, y[j]);
         }
         for (; e < e1; ++e) add4(s, row(e));
+        if (accumulate) {
+            float4 l = *out;
+            add4(l, s);
+            s = l;
+        }
         if (with_x) add4(s, reinterpret_cast<const float4*>(Lx + b * m * MS)[f]);
         if (4 * q + 3 < NC) {
             *out = s;
@@ -558,14 +590,18 @@ struct GemmShape {
 // Rows: a box holds MV = m (real) or 2m (CPLX: rows 2v and 2v + 1 the real and imaginary
 // planes of vector v) expansion rows of ms_of(P) slots; a product holds MV rows of
 // ys_of(P) slots.
-template <int P, typename T, bool CPLX = false>
+// ADD: the L2L of a level, Y = the locals: the product is added to the child's row as
+// add_local does (its X sum from Lx).  The vectors are dealt over blockIdx.y (a block a tile
+// with 16 vectors in turn took 80 us for levels of 24 to 104 tiles).
+template <int P, typename T, bool CPLX = false, bool ADD = false>
 __global__ void __launch_bounds__(256) m2l_gemm_kernel(const int32_t* __restrict__ tile_d,
                                                        const int64_t* __restrict__ tile_begin,
                                                        const int32_t* __restrict__ tile_count,
                                                        const int64_t* __restrict__ pair_e,
                                                        const int32_t* __restrict__ pair_src, int m,
                                                        const T* __restrict__ tab, const T* __restrict__ M,
-                                                       T* __restrict__ Y) {
+                                                       T* __restrict__ Y, DevPlan plan = {},
+                                                       const T* __restrict__ Lx = nullptr) {
     using S = GemmShape<P, T, CPLX>;
     constexpr int NC = S::NC, NE = S::NE, NCP = S::NCP, KC = S::KC;
     constexpr int JN = NCP / 16;
@@ -592,7 +628,7 @@ __global__ void __launch_bounds__(256) m2l_gemm_kernel(const int32_t* __restrict
     };
     if (kOneStage) stage_table(0, NE);
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    for (int v = 0; v < m; ++v) {
+    for (int v = blockIdx.y; v < m; v += gridDim.y) {
         const int vrow = CPLX ? 2 * v : v;
         T acc[4][JN];
 #pragma unroll
@@ -658,13 +694,17 @@ __global__ void __launch_bounds__(256) m2l_gemm_kernel(const int32_t* __restrict
             int pr = ty * 4 + i;
             if (pr >= cnt) continue;
             const int64_t e = pair_e ? pair_e[p0 + pr] : p0 + pr;
+            const bool x = ADD && x_of(plan, e, Lx);
 #pragma unroll
             for (int j = 0; j < JN; ++j) {
                 const int n = tx + 16 * j;
                 if (n < NE) {
                     const int plane = CPLX ? n / NC : 0, slot_ = CPLX ? n % NC : n;
-                    // read once by the reduce: stream past L2
-                    __stcs(Y + (e * mv + vrow + plane) * ys_of(P) + slot_, acc[i][j]);
+                    const int64_t at = (e * mv + vrow + plane) * ys_of(P) + slot_;
+                    if (ADD)
+                        add_local(Y + at, Lx + at, x, acc[i][j]);
+                    else  // read once by the reduce: stream past L2
+                        __stcs(Y + at, acc[i][j]);
                 }
             }
         }
