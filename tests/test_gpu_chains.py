@@ -1,5 +1,5 @@
 """Levels run as one chain launch (few children x vectors) and as launches over the device give
-the same floats: eight vectors move levels of a tree from one form to the other, at orders
+the same floats: eight vectors a pass move levels of a tree from one form to the other, at orders
 whose tables fit the chain and not (f64 p = 12); the Helmholtz form; both against the level
 calls, which run every level on its own."""
 import numpy as np
@@ -14,16 +14,16 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("p,n,leaf", [(3, 9000, 8), (6, 9000, 12), (8, 6000, 16), (12, 2500, 16)])
 def test_chain_and_wide_levels_same_floats(oracle, precision, p, n, leaf):
     x, q = oracle.point_sets("sphere", n, p)
-    b = F.FmmBuilder(p).max_points_per_leaf(leaf).precision(precision)
-    one = b.vectors(1).build(x)
-    want = one.evaluate(q)
-    lv = one.evaluate_levels(q)
-    assert np.array_equal(lv.potential, want.potential)
+    qs = np.stack([q * (v + 1.0) for v in range(8)], axis=1)
+    b = F.FmmBuilder(p).vectors(8).max_points_per_leaf(leaf).precision(precision)
+    one = b.vectors_per_pass(1).build(x)  # a vector a pass: small levels in chains
+    want = one.evaluate(qs)
     one.close()
-    many = b.vectors(8).build(x)
-    got = many.evaluate(np.stack([q * (v + 1.0) for v in range(8)], axis=1))
-    assert np.array_equal(got.potential[0], want.potential[0])
-    assert np.array_equal(got.potential[3], 4.0 * want.potential[0])  # a power of two: exact
+    many = b.vectors_per_pass(8).build(x)  # eight rows a child: the same levels wide
+    got = many.evaluate(qs)
+    assert np.array_equal(got.potential, want.potential)
+    lv = many.evaluate_levels(qs)
+    assert np.array_equal(lv.potential, want.potential)
     many.close()
 
 
@@ -32,14 +32,15 @@ def test_helmholtz_chain_and_wide_levels_same_floats(oracle, precision, p):
     x, q = oracle.point_sets("sphere", 5000, p)
     z = q + 1j * q[::-1]
     b = F.FmmBuilder(p).gradients().max_points_per_leaf(16).precision(precision)
-    one = b.vectors(1).build(x)
-    want = one.helmholtz_evaluate(5.0, z)
+    zs = np.stack([z * (v + 1.0) for v in range(5)], axis=1)
+    b = b.vectors(5)
+    one = b.vectors_per_pass(1).build(x)
+    want = one.helmholtz_evaluate(5.0, zs)
     one.close()
-    two = b.vectors(5).build(x)
-    got = two.helmholtz_evaluate(5.0, np.stack([z * (v + 1.0) for v in range(5)], axis=1))
-    scale = np.linalg.norm(want.potential)
-    # the near field and the tensor-core M2L of several vectors run on other kernels in the
-    # mixed form: 5e-6 there (f32 pairs), the same floats in f64
+    two = b.vectors_per_pass(5).build(x)
+    got = two.helmholtz_evaluate(5.0, zs)
+    # the near field of one vector runs on another kernel in the mixed form: 5e-6 there (f32
+    # pairs), the same floats in f64
     tol = 0.0 if precision == "f64" else 5e-6
-    assert np.linalg.norm(got.potential[0] - want.potential[0]) <= tol * scale
+    assert np.linalg.norm(got.potential - want.potential) <= tol * np.linalg.norm(want.potential)
     two.close()
