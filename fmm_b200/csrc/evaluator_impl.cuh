@@ -1375,16 +1375,15 @@ struct Evaluator final : EvaluatorBase {
 
     void leaf_far(int64_t r0, int64_t r1, int mode) {  // L2P / M2P of leaves [r0, r1)
         if (r1 <= r0) return;
-        const size_t smem = sizeof(T) == 8 ? NC * sizeof(T) : 0;
+        // a warp per P2P work item of these leaves (items are in leaf order); leaf_block
+        // threads a block
+        const int64_t i0 = std::lower_bound(item_leaf_h.begin(), item_leaf_h.end(), (int32_t)r0) - item_leaf_h.begin();
+        const int64_t i1 = std::lower_bound(item_leaf_h.begin(), item_leaf_h.end(), (int32_t)r1) - item_leaf_h.begin();
+        if (i1 <= i0) return;
+        const P2pItems it{items.leaf + i0, items.t0 + i0, i1 - i0};
+        const int wpb = leaf_block / 32;
+        const unsigned g = (unsigned)((it.count + wpb - 1) / wpb);
         if constexpr (kMixed) {
-            // a warp per P2P work item of these leaves (items are in leaf order); leaf_block
-            // threads a block
-            const int64_t i0 = std::lower_bound(item_leaf_h.begin(), item_leaf_h.end(), (int32_t)r0) - item_leaf_h.begin();
-            const int64_t i1 = std::lower_bound(item_leaf_h.begin(), item_leaf_h.end(), (int32_t)r1) - item_leaf_h.begin();
-            if (i1 <= i0) return;
-            const P2pItems it{items.leaf + i0, items.t0 + i0, i1 - i0};
-            const int wpb = leaf_block / 32;
-            const unsigned g = (unsigned)((it.count + wpb - 1) / wpb);
             const auto* tp = reinterpret_cast<const float4*>(tpos.ptr);
             const auto* Mf = reinterpret_cast<const float*>(M.ptr);
             const auto* Lf = reinterpret_cast<const float*>(Lc.ptr);
@@ -1394,14 +1393,16 @@ struct Evaluator final : EvaluatorBase {
             else
                 leaf_far_items_kernel<P, true><<<counted(g), leaf_block, 0, stream>>>(
                     dp, it, mode, m, tp, Mf, Lf, far_phi.as<double>(), far_g.as<double>());
-            return;
+        } else {
+            if (gradients)
+                leaf_far_f64_kernel<P, true><<<counted(g), leaf_block, 0, stream>>>(
+                    dp, it, mode, m, tpos.as<double4>(), M.as<double>(), Lc.as<double>(), far_phi.as<double>(),
+                    far_g.as<double>());
+            else
+                leaf_far_f64_kernel<P, false><<<counted(g), leaf_block, 0, stream>>>(
+                    dp, it, mode, m, tpos.as<double4>(), M.as<double>(), Lc.as<double>(), far_phi.as<double>(),
+                    far_g.as<double>());
         }
-        if (gradients)
-            leaf_far_kernel<P, T, true><<<counted((unsigned)(r1 - r0)), leaf_block, smem, stream>>>(
-                dp, r0, mode, m, tpos.as<T4>(), M.as<T>(), Lc.as<T>(), far_phi.as<double>(), far_g.as<double>());
-        else
-            leaf_far_kernel<P, T, false><<<counted((unsigned)(r1 - r0)), leaf_block, smem, stream>>>(
-                dp, r0, mode, m, tpos.as<T4>(), M.as<T>(), Lc.as<T>(), far_phi.as<double>(), far_g.as<double>());
     }
 
     template <int W, int KS>

@@ -149,43 +149,26 @@ __global__ void __launch_bounds__(32) expand_kernel(DevPlan plan, int64_t row_be
                 z = (p4.z - fc[2]) * finv;
             }
             for (int v = 0; v < m; ++v) Q[v * 32 + lane] = valid ? sq[(int64_t)v * plan.nsrc + si] : T(0);
-            if constexpr (!IRREG && sizeof(T) == 4) {  // f32: the rows on the packed pipe (leaf_far_x2.cuh)
-                RegularRows2<P> h;
-                h.init((float)x, (float)y, (float)z);
+            auto rows = [&](auto& h) {  // (pair rows, leaf_far_x2.cuh)
 #pragma unroll
                 for (int n = 0; n <= P; ++n) {
                     h.step(n);
 #pragma unroll
                     for (int mm = 0; mm <= n; ++mm) {
-                        S[slot(n, mm) * 32 + lane] = valid ? (T)h.c[mm].x : T(0);
-                        if (mm) S[slot(n, -mm) * 32 + lane] = valid ? (T)-h.c[mm].y : T(0);
+                        S[slot(n, mm) * 32 + lane] = valid ? h.c[mm].x : T(0);
+                        if (mm) S[slot(n, -mm) * 32 + lane] = valid ? -h.c[mm].y : T(0);
                     }
                 }
-            } else if (!IRREG) {
-                RegularRows<P, T> h;
+            };
+            if constexpr (!IRREG) {
+                RegularRows2<P, T> h;
                 h.init(x, y, z);
-#pragma unroll
-                for (int n = 0; n <= P; ++n) {
-                    h.step(n);
-#pragma unroll
-                    for (int mm = 0; mm <= n; ++mm) {
-                        S[slot(n, mm) * 32 + lane] = valid ? h.cre[mm] : T(0);
-                        if (mm) S[slot(n, -mm) * 32 + lane] = valid ? -h.cim[mm] : T(0);
-                    }
-                }
+                rows(h);
             } else {
-                IrregularRows<P, T> h;
-                T r2 = x * x + y * y + z * z;
+                IrregularRows2<P, T> h;
+                const T r2 = x * x + y * y + z * z;
                 h.init(x, y, z, valid ? T(1) / sqrt(r2) : T(0));
-#pragma unroll
-                for (int n = 0; n <= P; ++n) {
-                    h.step(n);
-#pragma unroll
-                    for (int mm = 0; mm <= n; ++mm) {
-                        S[slot(n, mm) * 32 + lane] = valid ? h.cre[mm] : T(0);
-                        if (mm) S[slot(n, -mm) * 32 + lane] = valid ? -h.cim[mm] : T(0);
-                    }
-                }
+                rows(h);
             }
             __syncwarp();
             int cnt = (int)((s1 - cb) < 32 ? (s1 - cb) : 32);
@@ -712,209 +695,12 @@ __global__ void __launch_bounds__(256) m2l_gemm_kernel(const int32_t* __restrict
 }
 
 // ---------------------------------------------------------------------------------
-// L2P (own local) then M2P (W list, by box index) for every target of a leaf.
-// Gradients by the ladder identities, contracted with shifted coefficients:
-//   (d/dx - i d/dy) phi = sum L_{k+1}^{mu+1} R_k^mu - conj(sum L_{k+1}^{mu-1} R_k^mu)
-//   d/dz phi = sum w_mu Re(L_{k+1}^mu R_k^mu)          (L2P; M2P uses M_{k-1}, sign -)
-// Results (phi_hat, g_hat in the leaf's units) go to the f64 far-field partials.
-// ---------------------------------------------------------------------------------
-// The weight 2 of the orders mu > 0 is applied once at the end: their terms add into
-// their own sums (f1, dz1), the mu = 0 terms (real harmonics: no imaginary part) into f0,
-// dz0, so a term costs two fused multiply-adds, not a product, a difference and a scaled add.
-template <int P, typename T, bool GRAD>
-__device__ __forceinline__ void l2p_eval(const T* L, T x, T y, T z, T& phi, T& gx, T& gy, T& gz) {
-    RegularRows<P, T> h;
-    h.init(x, y, z);
-    T f0 = T(0), f1 = T(0), dz0 = T(0), dz1 = T(0), are = T(0), aim = T(0);
-#pragma unroll
-    for (int k = 0; k <= P; ++k) {
-        h.step(k);
-#pragma unroll
-        for (int mu = 0; mu <= k; ++mu) {
-            Cx<T> c = coef_at(L, k, mu);
-            if (mu == 0) {
-                f0 += c.re * h.cre[0];
-            } else {
-                f1 += c.re * h.cre[mu];
-                f1 -= c.im * h.cim[mu];
-            }
-            if (GRAD && k < P) {
-                Cx<T> c1 = coef_at(L, k + 1, mu);
-                if (mu == 0) {
-                    dz0 += c1.re * h.cre[0];
-                } else {
-                    dz1 += c1.re * h.cre[mu];
-                    dz1 -= c1.im * h.cim[mu];
-                }
-                Cx<T> up = coef_at(L, k + 1, mu + 1);
-                are += up.re * h.cre[mu] - up.im * h.cim[mu];
-                aim += up.re * h.cim[mu] + up.im * h.cre[mu];
-                if (mu >= 1) {
-                    Cx<T> dn = coef_at(L, k + 1, mu - 1);
-                    are -= dn.re * h.cre[mu] - dn.im * h.cim[mu];
-                    aim += dn.re * h.cim[mu] + dn.im * h.cre[mu];  // minus conj
-                }
-            }
-        }
-    }
-    phi = f0 + T(2) * f1;
-    gx = are;
-    gy = -aim;
-    gz = dz0 + T(2) * dz1;
-}
-
-template <int P, typename T, bool GRAD>
-__device__ __forceinline__ void m2p_eval(const T* M, T x, T y, T z, T& phi, T& gx, T& gy, T& gz) {
-    constexpr int KMAX = GRAD ? P + 1 : P;
-    IrregularRows<P, T> h;
-    T r2 = x * x + y * y + z * z;
-    h.init(x, y, z, T(1) / sqrt(r2));
-    // the orders mu > 0 into their own sums, weighted 2 at the end (as l2p_eval)
-    T f0 = T(0), f1 = T(0), dz0 = T(0), dz1 = T(0), are = T(0), aim = T(0);
-#pragma unroll
-    for (int k = 0; k <= KMAX; ++k) {
-        h.step(k);
-#pragma unroll
-        for (int mu = 0; mu <= k; ++mu) {
-            if (k <= P) {
-                Cx<T> c = coef_at(M, k, mu);
-                if (mu == 0) {
-                    f0 += c.re * h.cre[0];
-                } else {
-                    f1 += c.re * h.cre[mu];
-                    f1 -= c.im * h.cim[mu];
-                }
-            }
-            if (GRAD && k >= 1) {
-                Cx<T> c1 = coef_at(M, k - 1, mu);
-                if (mu == 0) {
-                    dz0 -= c1.re * h.cre[0];
-                } else {
-                    dz1 -= c1.re * h.cre[mu];
-                    dz1 += c1.im * h.cim[mu];
-                }
-                if (mu <= k - 2) {
-                    Cx<T> up = coef_at(M, k - 1, mu + 1);
-                    are += up.re * h.cre[mu] - up.im * h.cim[mu];
-                    aim += up.re * h.cim[mu] + up.im * h.cre[mu];
-                }
-                if (mu >= 1) {
-                    Cx<T> dn = coef_at(M, k - 1, mu - 1);
-                    are -= dn.re * h.cre[mu] - dn.im * h.cim[mu];
-                    aim += dn.re * h.cim[mu] + dn.im * h.cre[mu];
-                }
-            }
-        }
-    }
-    phi = f0 + T(2) * f1;
-    gx = are;
-    gy = -aim;
-    gz = dz0 + T(2) * dz1;
-}
-
-// mode: bit 0 L2P, bit 1 M2P, bit 2 add into far_phi / far_g (else overwrite them).
-// The evaluation runs mode 3; the level calls run 5 (L2P) then 6 (M2P) on stores that
-// start at zero, which gives the same floats.
-template <int P, typename T, bool GRAD>
-__global__ void __launch_bounds__(128) leaf_far_kernel(DevPlan plan, int64_t leaf0, int mode, int m,
-                                                      const typename Vec4<T>::type* __restrict__ tpos,
-                                                      const T* __restrict__ M, const T* __restrict__ Lc,
-                                                      double* __restrict__ far_phi, double* __restrict__ far_g) {
-    constexpr int NC = nc_of(P);
-    // f32: the expansions are read straight from global memory (every thread reads the same
-    // coefficient at the same time: one broadcast through L1, no block barrier); f64 stages
-    // each expansion in shared memory (measured faster for 8-byte coefficients)
-    constexpr bool kStage = sizeof(T) == 8;
-    extern __shared__ unsigned char smem_raw[];
-    T* C = reinterpret_cast<T*>(smem_raw);  // [NC] when staged
-    const int64_t leaf = leaf0 + blockIdx.x;
-    const int box = plan.leaf_box[leaf];
-    const int64_t t0 = plan.tgt_start[leaf], t1 = plan.tgt_start[leaf + 1];
-    if (t1 == t0) return;
-    const int64_t w0 = plan.w_row[leaf], w1 = (mode & 2) ? plan.w_row[leaf + 1] : plan.w_row[leaf];
-    const int64_t nt = plan.ntgt;
-    for (int v = 0; v < m; ++v) {
-        for (int64_t tb = t0; tb < t1; tb += blockDim.x) {
-            int64_t t = tb + threadIdx.x;
-            bool valid = t < t1;
-            T ux = T(0), uy = T(0), uz = T(0);
-            if (valid) {
-                auto p4 = tpos[t];
-                ux = p4.x;
-                uy = p4.y;
-                uz = p4.z;
-            }
-            double fphi = 0.0, fg[3] = {0.0, 0.0, 0.0};
-            if ((mode & 4) && valid) {
-                fphi = far_phi[(int64_t)v * nt + t];
-                if (GRAD)
-                    for (int k = 0; k < 3; ++k) fg[k] = far_g[((int64_t)v * nt + t) * 3 + k];
-            }
-            // L2P, unit frame
-            if (mode & 1) {
-                const T* Lb = Lc + ((int64_t)box * m + v) * ms_of(P);
-                if (kStage) {
-                    for (int k = threadIdx.x; k < NC; k += blockDim.x) C[k] = Lb[k];
-                    __syncthreads();
-                    Lb = C;
-                }
-                if (valid) {
-                    T ph, gx, gy, gz;
-                    l2p_eval<P, T, GRAD>(Lb, ux, uy, uz, ph, gx, gy, gz);
-                    fphi = (mode & 4) ? fphi + (double)ph : (double)ph;
-                    if (GRAD) {
-                        fg[0] = (mode & 4) ? fg[0] + (double)gx : (double)gx;
-                        fg[1] = (mode & 4) ? fg[1] + (double)gy : (double)gy;
-                        fg[2] = (mode & 4) ? fg[2] + (double)gz : (double)gz;
-                    }
-                }
-                if (kStage) __syncthreads();
-            }
-            // M2P over the W list, frame (c(s|t), r(s|t))
-            for (int64_t e = w0; e < w1; ++e) {
-                int s = plan.w_col[e];
-                const T* Mb = M + ((int64_t)s * m + v) * ms_of(P);
-                if (kStage) {
-                    for (int k = threadIdx.x; k < NC; k += blockDim.x) C[k] = Mb[k];
-                    __syncthreads();
-                    Mb = C;
-                }
-                if (valid) {
-                    T c[3], r;
-                    rel_frame<T>(plan, s, box, c, r);
-                    T rinv = T(1) / r;
-                    T ph, gx, gy, gz;
-                    m2p_eval<P, T, GRAD>(Mb, (ux - c[0]) * rinv, (uy - c[1]) * rinv, (uz - c[2]) * rinv, ph, gx,
-                                         gy, gz);
-                    fphi += (double)(ph * rinv);
-                    if (GRAD) {
-                        T r2inv = rinv * rinv;
-                        fg[0] += (double)(gx * r2inv);
-                        fg[1] += (double)(gy * r2inv);
-                        fg[2] += (double)(gz * r2inv);
-                    }
-                }
-                if (kStage) __syncthreads();
-            }
-            if (valid) {
-                far_phi[(int64_t)v * nt + t] = fphi;
-                if (GRAD) {
-                    double* g = far_g + ((int64_t)v * nt + t) * 3;
-                    g[0] = fg[0];
-                    g[1] = fg[1];
-                    g[2] = fg[2];
-                }
-            }
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------------
 // L2P + M2P of the potentials for several charge vectors (f32, m > 1): the harmonics of a
 // target are formed once per W entry (and once for L2P) and dotted with VB vectors'
-// expansions, which are consecutive rows of ms_of(P) floats.  Per vector the terms are
-// those of l2p_eval / m2p_eval, with the harmonic rows on the packed f32x2 pipe and each
-// order mu > 0 one packed fused multiply-add (real and imaginary products summed apart).
+// expansions, which are consecutive rows of ms_of(P) floats, the harmonic rows on the packed
+// f32x2 pipe and each order mu > 0 one packed fused multiply-add (real and imaginary products
+// summed apart).  (Rows read 16 bytes at a time, a group of degrees in registers, were slower:
+// 2.12 against 1.72 ms for 700,000 points with 16 vectors at p = 6, with 168 registers a thread.)
 template <int P, int VB>
 __device__ __forceinline__ void l2p_eval_mv(const float* L, int nb, float x, float y, float z, float (&f)[VB]) {
     constexpr int MS = ms_of(P);
@@ -1034,12 +820,13 @@ __device__ __forceinline__ void item_shape(const P2pItems& items, int64_t item, 
     ni = ns = (int)(r < 32 ? r : 32);
 }
 
-// L2P + M2P of the f32 form over P2P work items: a warp per item (up to 32 targets of one
-// leaf, lane = target), any number of warps a block.  Each target sums the terms of
-// leaf_far_kernel<P, float, GRAD> in the same order (the compiler may contract products
-// into fmas differently, so the last bits can differ); what changes is the occupancy: a
-// block per leaf holds every thread of its block while a leaf of few targets keeps one
-// warp busy, a warp per item leaves no idle warp resident.  leaf_far_mv_items_kernel forms
+// L2P (own local) then M2P (W list, by box index) for every target of a leaf, over the P2P
+// work items: a warp per item (up to 32 targets of one leaf, lane = target), any number of
+// warps a block; a block per leaf held its whole block's registers while a leaf of few targets
+// kept one warp busy.  Results (phi_hat, g_hat in the leaf's units) go to the f64 far-field
+// partials.  mode: bit 0 L2P, bit 1 M2P, bit 2 add into far_phi / far_g (else overwrite them):
+// the evaluation runs mode 3; the level calls run 5 (L2P) then 6 (M2P) on stores that start
+// at zero, which gives the same floats.  leaf_far_mv_items_kernel forms
 // each target's harmonics once for up to VB vectors (l2p_eval_mv / m2p_eval_mv).
 // The gradient form is held to 96 registers up to p = 8 (21 warps an SM, no spills) and to
 // 168 above (12 warps an SM; no spills to p = 12).
@@ -1073,7 +860,7 @@ __global__ void __launch_bounds__(128, P <= 8 ? 5 : 3) leaf_far_items_kernel(Dev
         }
         if (mode & 1) {
             float ph, gx, gy, gz;
-            l2p_x2<P>(Lc + ((int64_t)box * m + v) * ms_of(P), ux, uy, uz, ph, gx, gy, gz);
+            l2p_x2<P, float>(Lc + ((int64_t)box * m + v) * ms_of(P), ux, uy, uz, ph, gx, gy, gz);
             fphi = (mode & 4) ? fphi + (double)ph : (double)ph;
             fg[0] = (mode & 4) ? fg[0] + (double)gx : (double)gx;
             fg[1] = (mode & 4) ? fg[1] + (double)gy : (double)gy;
@@ -1085,7 +872,7 @@ __global__ void __launch_bounds__(128, P <= 8 ? 5 : 3) leaf_far_items_kernel(Dev
             rel_frame<float>(plan, s, box, c, r);
             const float rinv = 1.0f / r;
             float ph, gx, gy, gz;
-            m2p_x2<P>(M + ((int64_t)s * m + v) * ms_of(P), (ux - c[0]) * rinv, (uy - c[1]) * rinv,
+            m2p_x2<P, float>(M + ((int64_t)s * m + v) * ms_of(P), (ux - c[0]) * rinv, (uy - c[1]) * rinv,
                       (uz - c[2]) * rinv, ph, gx, gy, gz);
             fphi += (double)(ph * rinv);
             const float r2inv = rinv * rinv;
@@ -1143,6 +930,78 @@ __global__ void __launch_bounds__(128) leaf_far_mv_items_kernel(DevPlan plan, P2
 #pragma unroll
         for (int b = 0; b < VB; ++b)
             if (b < nb) far_phi[(int64_t)(v0 + b) * nt + t] = fphi[b];
+    }
+}
+
+// The f64 form: a warp per item, its lanes over the item's (target, vector) pairs, target
+// fastest, so that a leaf of five targets and four vectors keeps 20 lanes busy (a thread a
+// target with the vectors in turn, the expansions staged in shared memory behind two block
+// barriers each, kept 5).  Coefficients are read straight from global memory, the same value
+// for every lane of one vector.  Each evaluation's sums do not depend on the other lanes.
+// Bound by the coefficients' loads and the FP64 pipe.  Measured: 41,017 targets x 4 vectors at
+// p = 10 (5 targets a leaf) 0.89 -> 0.27 ms, 1e6 targets at p = 8 0.25 -> 0.10.
+template <int P, bool GRAD>
+__global__ void __launch_bounds__(128) leaf_far_f64_kernel(DevPlan plan, P2pItems items, int mode, int m,
+                                                          const double4* __restrict__ tpos,
+                                                          const double* __restrict__ M, const double* __restrict__ Lc,
+                                                          double* __restrict__ far_phi, double* __restrict__ far_g) {
+    const int64_t item = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (item >= items.count) return;
+    const int leaf = items.leaf[item];
+    const int64_t t0 = items.t0[item], t1 = plan.tgt_start[leaf + 1];
+    const int ni = t1 - t0 < 32 ? (int)(t1 - t0) : 32;
+    const int box = plan.leaf_box[leaf];
+    const int64_t w0 = plan.w_row[leaf], w1 = (mode & 2) ? plan.w_row[leaf + 1] : plan.w_row[leaf];
+    const int64_t nt = plan.ntgt;
+    for (int u = threadIdx.x & 31; u < ni * m; u += 32) {
+        const int v = u / ni;
+        const int64_t t = t0 + u % ni, at = (int64_t)v * nt + t;
+        const double4 p4 = tpos[t];
+        double fphi = 0.0, fg[3] = {0.0, 0.0, 0.0};
+        if (mode & 4) {
+            fphi = far_phi[at];
+            if (GRAD)
+                for (int k = 0; k < 3; ++k) fg[k] = far_g[at * 3 + k];
+        }
+        if (mode & 1) {
+            const double* L = Lc + ((int64_t)box * m + v) * ms_of(P);
+            double ph, gx = 0.0, gy = 0.0, gz = 0.0;
+            if constexpr (GRAD) {
+                l2p_x2<P, double>(L, p4.x, p4.y, p4.z, ph, gx, gy, gz);
+            } else {
+                RegularRows2<P, double> h;
+                h.init(p4.x, p4.y, p4.z);
+                ph = phi_eval<P>(h, L);
+            }
+            fphi += ph;
+            fg[0] += gx;
+            fg[1] += gy;
+            fg[2] += gz;
+        }
+        for (int64_t e = w0; e < w1; ++e) {
+            const int s = plan.w_col[e];
+            double c[3], r;
+            rel_frame<double>(plan, s, box, c, r);
+            const double rinv = 1.0 / r;
+            const double x = (p4.x - c[0]) * rinv, y = (p4.y - c[1]) * rinv, z = (p4.z - c[2]) * rinv;
+            const double* Mb = M + ((int64_t)s * m + v) * ms_of(P);
+            double ph, gx = 0.0, gy = 0.0, gz = 0.0;
+            if constexpr (GRAD) {
+                m2p_x2<P, double>(Mb, x, y, z, ph, gx, gy, gz);
+            } else {
+                IrregularRows2<P, double> h;
+                h.init(x, y, z, 1.0 / sqrt(x * x + y * y + z * z));
+                ph = phi_eval<P>(h, Mb);
+            }
+            fphi += ph * rinv;
+            const double r2inv = rinv * rinv;
+            fg[0] += gx * r2inv;
+            fg[1] += gy * r2inv;
+            fg[2] += gz * r2inv;
+        }
+        far_phi[at] = fphi;
+        if (GRAD)
+            for (int k = 0; k < 3; ++k) far_g[at * 3 + k] = fg[k];
     }
 }
 
