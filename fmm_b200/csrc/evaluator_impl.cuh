@@ -39,7 +39,7 @@ struct HhState {
     bool built = false;
     // the mixed form's tensor-core M2L (p <= 10): tiles over every level, (level, offset,
     // half) as the table index, the table images, and the multipoles' tensor maps
-    DevBuf tc_d, tc_begin, tc_count, tc_img;
+    DevBuf tc_d, tc_begin, tc_count, tc_cta, tc_img;
     int64_t tc_ntiles = 0;
     CUtensorMap mmap{}, vmap{};
 };
@@ -94,6 +94,12 @@ struct Evaluator final : EvaluatorBase {
     DevBuf tc2_tile_d, tc2_tile_begin, tc2_tile_count, tc2_ltile_d, tc2_ltile_begin, tc2_ltile_count;
     std::vector<int64_t> tc2_lvl_tiles;
     int64_t tc2_ntiles = 0;
+    DevBuf tc_cta, tc2_cta;  // the CTAs' tile ranges of the two all-level lists
+    // the ranges of a launch over `d`'s tiles (grid of min(tiles, num_sms) CTAs)
+    void upload_ranges(DevBuf& b, const std::vector<int32_t>& d) {
+        const int64_t n = (int64_t)d.size();
+        b.upload(tc_tile_ranges(d, std::max<int64_t>(1, std::min<int64_t>(n, num_sms))));
+    }
     int num_sms = 148;
     // fused tensor-core M2L: per level, chunks of consecutive target boxes cut into tiles
     // of one offset (pairs in (chunk, offset, target) order), CTA c of level l taking the
@@ -454,6 +460,7 @@ struct Evaluator final : EvaluatorBase {
             tc_halves(all, nullptr);
             tc_halves(lvl, &tc_lvl_tiles);
             tc_ntiles = (int64_t)all.d.size();
+            upload_ranges(tc_cta, all.d);
             tc_tile_d.upload(all.d);
             tc_tile_begin.upload(all.begin);
             tc_tile_count.upload(all.count);
@@ -469,6 +476,7 @@ struct Evaluator final : EvaluatorBase {
             tc_halves(all2, nullptr);
             tc_halves(lvl2, &tc2_lvl_tiles);
             tc2_ntiles = (int64_t)all2.d.size();
+            upload_ranges(tc2_cta, all2.d);
             tc2_tile_d.upload(all2.d);
             tc2_tile_begin.upload(all2.begin);
             tc2_tile_count.upload(all2.count);
@@ -554,7 +562,7 @@ struct Evaluator final : EvaluatorBase {
                 const unsigned grid = (unsigned)std::min<int64_t>(c.tc_nt, num_sms);
                 m2l_tc_kernel<P><<<counted(grid), 32 * kTcWarps, TcTs<P>::SMEM, stream>>>(
                     ck_tc_d.as<int32_t>() + c.tc_t0, ck_tc_begin.as<int64_t>() + c.tc_t0,
-                    ck_tc_count.as<int32_t>() + c.tc_t0, c.tc_nt, ck_pair_src.as<int32_t>() + c.base, m,
+                    ck_tc_count.as<int32_t>() + c.tc_t0, c.tc_nt, nullptr, ck_pair_src.as<int32_t>() + c.base, m,
                     tc_bimg.as<uint32_t>(), mmap, vmap, reinterpret_cast<float*>(Y.ptr), tc_error.as<int>());
             }
             return;
@@ -1074,7 +1082,7 @@ struct Evaluator final : EvaluatorBase {
                                &fu_tile_np, &fu_cta, &fu_pair_src, &fu_pair_tgt, &fu_img, &ck_tc_d, &ck_tc_begin,
                                &ck_tc_count, &ck_s_d, &ck_s_begin, &ck_s_count, &ck_pair_src, &st_rowpair,
                                &st_xy, &st_zz, &st_idx, &close_w, &close_acc, &close_src32, &up_off, &down_off,
-                               &m2m_start_d};
+                               &m2m_start_d, &tc_cta, &tc2_cta};
         size_t s = 0;
         for (auto* b : all) s += b->bytes;
         return s;
@@ -1333,15 +1341,16 @@ struct Evaluator final : EvaluatorBase {
                 const DevBuf& tn = l < 0 ? (alt ? tc2_tile_count : tc_tile_count) : (alt ? tc2_ltile_count : tc_ltile_count);
                 if (nt == 0) return;
                 const unsigned grid = (unsigned)std::min<int64_t>(nt, num_sms);
+                const int64_t* ranges = l < 0 ? (alt ? tc2_cta : tc_cta).as<int64_t>() : nullptr;
                 if (alt)
                     m2l_tc_kernel<P, false, kTcAlt><<<counted(grid), 32 * kTcWarps, TcTs<P, false, kTcAlt>::SMEM,
                                                       stream>>>(
-                        td.as<int32_t>() + t0, tb.as<int64_t>() + t0, tn.as<int32_t>() + t0, nt,
+                        td.as<int32_t>() + t0, tb.as<int64_t>() + t0, tn.as<int32_t>() + t0, nt, ranges,
                         tc_pair_src.as<int32_t>(), m, tc_bimg.as<uint32_t>(), mmap, vmap,
                         reinterpret_cast<float*>(Y.ptr), tc_error.as<int>());
                 else
                     m2l_tc_kernel<P><<<counted(grid), 32 * kTcWarps, TcTs<P>::SMEM, stream>>>(
-                        td.as<int32_t>() + t0, tb.as<int64_t>() + t0, tn.as<int32_t>() + t0, nt,
+                        td.as<int32_t>() + t0, tb.as<int64_t>() + t0, tn.as<int32_t>() + t0, nt, ranges,
                         tc_pair_src.as<int32_t>(), m, tc_bimg.as<uint32_t>(), mmap, vmap,
                         reinterpret_cast<float*>(Y.ptr), tc_error.as<int>());
             }
@@ -1627,6 +1636,7 @@ struct Evaluator final : EvaluatorBase {
             for (int l = 0; l < plan.nlevels; ++l)
                 for (int64_t i = lstart[l]; i < lstart[l + 1]; ++i) lvl.d[i] += (l - 2) * 316 * 2;
             hh.tc_ntiles = (int64_t)lvl.d.size();
+            upload_ranges(hh.tc_cta, lvl.d);
             hh.tc_d.upload(lvl.d);
             hh.tc_begin.upload(lvl.begin);
             hh.tc_count.upload(lvl.count);
@@ -1708,7 +1718,7 @@ struct Evaluator final : EvaluatorBase {
                 const unsigned grid = (unsigned)std::min<int64_t>(hh.tc_ntiles, num_sms);
                 m2l_tc_kernel<P, true><<<counted(grid), 32 * kTcWarps, TcTs<P, true>::SMEM, stream>>>(
                     hh.tc_d.as<int32_t>(), hh.tc_begin.as<int64_t>(), hh.tc_count.as<int32_t>(), hh.tc_ntiles,
-                    pair_src.as<int32_t>(), 2 * m, hh.tc_img.as<uint32_t>(), hh.mmap, hh.vmap,
+                    hh.tc_cta.as<int64_t>(), pair_src.as<int32_t>(), 2 * m, hh.tc_img.as<uint32_t>(), hh.mmap, hh.vmap,
                     reinterpret_cast<float*>(hh.Y.ptr), tc_error.as<int>());
             }
         } else {

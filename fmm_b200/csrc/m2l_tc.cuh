@@ -124,8 +124,9 @@ __device__ __forceinline__ void umma_commit(uint32_t mbar) {
                  : "memory");
 }
 
-// Persistent, warp-specialised form.  CTA c takes the contiguous range of tiles
-// [c T / G, (c + 1) T / G) of the offset-sorted tile list.  The table of the current
+// Persistent, warp-specialised form.  CTA c takes a contiguous range of the offset-sorted tile
+// list: cta_tiles[c] .. cta_tiles[c + 1] when given (tc_tile_ranges), else an equal share.  The
+// table of the current
 // offset lives in tensor memory as the MMA's A operand (M = 128 lanes = output slots,
 // K = input slots in columns; hi and lo parts), so the MMA is D[slot][pair] = A_d . X^T
 // with the gathered multipoles X as the shared-memory B operand (N = NT pairs,
@@ -141,8 +142,9 @@ __device__ __forceinline__ void umma_commit(uint32_t mbar) {
 //     misses;
 //   warps 8-15 (converters): wait raw_full, split the raw rows into X stage k&1
 //     (x = hi + lo in tf32, 128-byte swizzled) once MMA(k-2) has released it
-//     (empty[k&1]), signal full[k&1] and raw_empty; warps 8-11 also replace the table in
-//     tensor memory when the offset changes, after MMA(k-1) has read the old one;
+//     (empty[k&1]), signal full[k&1] and raw_empty; they also replace the table in tensor
+//     memory when the offset changes (a warp a lane quarter of the hi or lo part), after
+//     MMA(k-1) has read the old one;
 //   warp 16, one thread (MMA): waits full[k&1], the table and the accumulator k&1
 //     (acc_empty, released by the epilogue of tile k-2), issues the 3 x KSTEPS MMAs
 //     and commits to empty[k&1] and acc_full[k&1];
@@ -254,11 +256,28 @@ __device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
+// The converters' chunks of a tile: 256 threads cover ROWS rows in N steps, the smallest N that
+// makes that a whole number of rows, and a multiple of 8 rows.
+constexpr int tc_convert_period(int quads) {
+    int n = 1;
+    while ((32 * kTcProd * n) % quads != 0 || (32 * kTcProd * n / quads) % 8 != 0) ++n;
+    return n;
+}
+template <int NT, int KP>
+struct TcConvert {
+    static constexpr int QUADS = KP / 4;  // chunks a row
+    static constexpr int N = tc_convert_period(QUADS);
+    static constexpr int ROWS = 32 * kTcProd * N / QUADS;
+    static constexpr int STEPS = (NT * QUADS + 32 * kTcProd - 1) / (32 * kTcProd);
+    static constexpr bool PART = NT * QUADS % (32 * kTcProd) != 0;  // the last step is not full
+};
+
 template <int P, bool CPLX = false, int NTA = 0>
 __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t* __restrict__ tile_d,
                                                                   const int64_t* __restrict__ tile_begin,
                                                                   const int32_t* __restrict__ tile_count,
                                                                   int64_t ntiles,
+                                                                  const int64_t* __restrict__ cta_tiles,
                                                                   const int32_t* __restrict__ pair_src, int m,
                                                                   const uint32_t* __restrict__ timg,
                                                                   const __grid_constant__ CUtensorMap mmap,
@@ -274,8 +293,8 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
     __shared__ uint64_t bar_full[2], bar_empty[2], bar_accf[2], bar_acce[2], bar_table, bar_rfull[RS], bar_rempty[RS];
     __shared__ uint32_t tmem_base;
     __shared__ int abort_flag;
-    const int64_t i0 = (int64_t)blockIdx.x * ntiles / gridDim.x;
-    const int64_t i1 = (int64_t)(blockIdx.x + 1) * ntiles / gridDim.x;
+    const int64_t i0 = cta_tiles ? cta_tiles[blockIdx.x] : (int64_t)blockIdx.x * ntiles / gridDim.x;
+    const int64_t i1 = cta_tiles ? cta_tiles[blockIdx.x + 1] : (int64_t)(blockIdx.x + 1) * ntiles / gridDim.x;
     if (i0 >= i1) return;
     const int64_t ntile = i1 - i0;
 
@@ -295,7 +314,7 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
             mbar_init(smem_u32(&bar_rfull[b]), 1);
             mbar_init(smem_u32(&bar_rempty[b]), kTcProd);
         }
-        mbar_init(smem_u32(&bar_table), 4);
+        mbar_init(smem_u32(&bar_table), kTcProd);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
@@ -327,13 +346,8 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
         const int ppt = NT / m;            // pairs a tile holds
         const uint32_t tx = blocks ? (uint32_t)(ppt * m * KP * 4) : (uint32_t)S::X_BYTES;
         int64_t issued = 0;
-        for (int64_t k = 0; k < ntile && !warp_aborted(); ++k) {
-            const int64_t it = i0 + k;
-            const int rs = (int)(k % RS);
-            const int64_t p0 = tile_begin[it];
-            const int ncol = tile_count[it] * m;
-            // rows past the tile's columns fetch row 0 (their products are never stored)
-            int r[4];
+        // a tile's rows in r: rows past its columns fetch row 0 (their products are never stored)
+        auto rows = [&](int64_t p0, int ncol, int (&r)[4]) {
             if (blocks) {
                 r[0] = (lane < ppt && lane * m < ncol) ? pair_src[p0 + lane] * m : 0;
             } else if (m == 1) {  // the common case without the divisions
@@ -348,6 +362,20 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
                     const int c = 4 * lane + j;
                     r[j] = (c < ncol) ? pair_src[p0 + c / m] * m + c % m : 0;
                 }
+            }
+        };
+        // the tile's place is read two tiles ahead and its rows one ahead: each is an L2 load
+        // that would else stand in the tile's way
+        int r[4], rn[4] = {0, 0, 0, 0};
+        rows(tile_begin[i0], tile_count[i0] * m, r);
+        int64_t p1 = ntile > 1 ? tile_begin[i0 + 1] : 0;
+        int n1 = ntile > 1 ? tile_count[i0 + 1] * m : 0;
+        for (int64_t k = 0; k < ntile && !warp_aborted(); ++k) {
+            const int rs = (int)(k % RS);
+            if (k + 1 < ntile) rows(p1, n1, rn);
+            if (k + 2 < ntile) {
+                p1 = tile_begin[i0 + k + 2];
+                n1 = tile_count[i0 + k + 2] * m;
             }
             if (k >= RS && !warp_wait(&bar_rempty[rs], (uint32_t)(((k - RS) / RS) & 1))) {
                 if (lane == 0) give_up();
@@ -364,6 +392,8 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
                             smem_u32(&bar_rfull[rs]));
             }
             issued = k + 1;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) r[j] = rn[j];
         }
         // on a give-up, the gathers still in flight land before the shared memory is released
         if (lane == 0 && *abort)
@@ -374,9 +404,16 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
         // ---------------- converters ----------------
         const int pw = warp - kTcProd;
         const int ctid = tid - 32 * kTcProd;  // 0 .. 255
-        const uint32_t* img_prev = nullptr;
+        using CV = TcConvert<NT, KP>;
+        uint32_t cv_off[CV::N];
+#pragma unroll
+        for (int j = 0; j < CV::N; ++j) {
+            const int c = ctid + j * 32 * kTcProd;
+            cv_off[j] = sw128_offset(c / (KP / 4), 4 * (c % (KP / 4)), NT);
+        }
+        int d = tile_d[i0], d_prev = -1;  // (the next tile's read ahead, in every role)
         for (int64_t k = 0; k < ntile && !warp_aborted(); ++k) {
-            const int64_t it = i0 + k;
+            const int d_next = k + 1 < ntile ? tile_d[i0 + k + 1] : 0;
             const int st = (int)(k & 1);
             unsigned char* xh = xbuf + (size_t)st * 2 * S::X_BYTES;
             unsigned char* xl = xh + S::X_BYTES;
@@ -388,69 +425,79 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
                 if (lane == 0) give_up();
                 break;
             }
-            // raw [NT][KP] -> hi / lo, four consecutive slots (one 16-byte chunk) at a time
-#pragma unroll 4
-            for (int c = ctid; c < NT * KP / 4; c += 32 * kTcProd) {
-                const int row = c / (KP / 4), k4 = 4 * (c % (KP / 4));
-                const float4 x = raw[c];
-                uint4 hi, lo;
-                hi.x = cvt_tf32(x.x);
-                hi.y = cvt_tf32(x.y);
-                hi.z = cvt_tf32(x.z);
-                hi.w = cvt_tf32(x.w);
-                lo.x = cvt_tf32(x.x - __uint_as_float(hi.x));
-                lo.y = cvt_tf32(x.y - __uint_as_float(hi.y));
-                lo.z = cvt_tf32(x.z - __uint_as_float(hi.z));
-                lo.w = cvt_tf32(x.w - __uint_as_float(hi.w));
-                const uint32_t off = sw128_offset(row, k4, NT);
-                *reinterpret_cast<uint4*>(xh + off) = hi;
-                *reinterpret_cast<uint4*>(xl + off) = lo;
-            }
+            // raw [NT][KP] -> hi / lo, four consecutive slots (one 16-byte chunk) at a time.  A
+            // thread's chunks c = ctid + 256 i repeat their place in a row, and their swizzle,
+            // every CV::ROWS rows (a multiple of 8), so its CV::N offsets are formed once and a
+            // chunk costs its loads, its rounding and its stores.  (The hand-offs between the roles
+            // bound the kernel more than any one role's work: without its conversions a sphere of
+            // 1e6 points at p = 8 took 0.187 instead of 0.207 ms, without gathers, conversions and
+            // stores 0.170; with this and the tiles' places read ahead 0.199, and the M2L of 4e6
+            // points 0.74 -> 0.66, of a batch with 16 vectors at p = 6 5.0 -> 4.5.)
+#pragma unroll
+            for (int g0 = 0; g0 < CV::STEPS; g0 += CV::N)
+#pragma unroll
+                for (int j = 0; j < CV::N && g0 + j < CV::STEPS; ++j) {
+                    const int c = ctid + (g0 + j) * 32 * kTcProd;
+                    if (CV::PART && c >= NT * KP / 4) break;
+                    const float4 x = raw[c];
+                    uint4 hi, lo;
+                    hi.x = tf32_round_bits(__float_as_uint(x.x));
+                    hi.y = tf32_round_bits(__float_as_uint(x.y));
+                    hi.z = tf32_round_bits(__float_as_uint(x.z));
+                    hi.w = tf32_round_bits(__float_as_uint(x.w));
+                    lo.x = tf32_round_bits(__float_as_uint(x.x - __uint_as_float(hi.x)));
+                    lo.y = tf32_round_bits(__float_as_uint(x.y - __uint_as_float(hi.y)));
+                    lo.z = tf32_round_bits(__float_as_uint(x.z - __uint_as_float(hi.z)));
+                    lo.w = tf32_round_bits(__float_as_uint(x.w - __uint_as_float(hi.w)));
+                    const uint32_t off = cv_off[j] + (uint32_t)(g0 / CV::N) * CV::ROWS * 128u;
+                    *reinterpret_cast<uint4*>(xh + off) = hi;
+                    *reinterpret_cast<uint4*>(xl + off) = lo;
+                }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(smem_u32(&bar_full[st]));
                 mbar_arrive(smem_u32(&bar_rempty[rs]));
             }
-            // the table of tile k (warps 8-11, one per lane quarter), once MMA(k-1) is done
-            const uint32_t* img = timg + (size_t)tile_d[it] * S::IMG_WORDS;
-            if (pw < 4 && img != img_prev) {
+            // the table of tile k (a warp a lane quarter and part), once MMA(k-1) is done
+            if (d != d_prev) {
+                const uint32_t* img = timg + (size_t)d * S::IMG_WORDS;
                 if (k >= 1 && !warp_wait(&bar_empty[(k - 1) & 1], (uint32_t)(((k - 1) >> 1) & 1))) {
                     if (lane == 0) give_up();
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;");
+                const int part = pw >> 2, quarter = pw & 3;
 #pragma unroll 1
-                for (int part = 0; part < 2; ++part)
-#pragma unroll 1
-                    for (int k0 = 0; k0 < S::KP; k0 += 48) {
-                        uint4 u[12];
-                        const uint4* row =
-                            reinterpret_cast<const uint4*>(img + ((size_t)part * 128 + 32 * pw + lane) * S::KP + k0);
+                for (int k0 = 0; k0 < S::KP; k0 += 48) {
+                    uint4 u[12];
+                    const uint4* row =
+                        reinterpret_cast<const uint4*>(img + ((size_t)part * 128 + 32 * quarter + lane) * S::KP + k0);
 #pragma unroll
-                        for (int q = 0; q < 12; ++q) u[q] = (k0 + 4 * q < S::KP) ? __ldg(row + q) : make_uint4(0, 0, 0, 0);
+                    for (int q = 0; q < 12; ++q) u[q] = (k0 + 4 * q < S::KP) ? __ldg(row + q) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-                        for (int h = 0; h < 3; ++h) {
-                            if (k0 + 16 * h >= S::KP) break;
-                            uint32_t r16[16];
+                    for (int h = 0; h < 3; ++h) {
+                        if (k0 + 16 * h >= S::KP) break;
+                        uint32_t r16[16];
 #pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                r16[4 * q] = u[4 * h + q].x;
-                                r16[4 * q + 1] = u[4 * h + q].y;
-                                r16[4 * q + 2] = u[4 * h + q].z;
-                                r16[4 * q + 3] = u[4 * h + q].w;
-                            }
-                            tmem_st16(tmem + ((uint32_t)(32 * pw) << 16) +
-                                          (uint32_t)((part ? S::COL_ALO : S::COL_AHI) + k0 + 16 * h),
-                                      r16);
+                        for (int q = 0; q < 4; ++q) {
+                            r16[4 * q] = u[4 * h + q].x;
+                            r16[4 * q + 1] = u[4 * h + q].y;
+                            r16[4 * q + 2] = u[4 * h + q].z;
+                            r16[4 * q + 3] = u[4 * h + q].w;
                         }
+                        tmem_st16(tmem + ((uint32_t)(32 * quarter) << 16) +
+                                      (uint32_t)((part ? S::COL_ALO : S::COL_AHI) + k0 + 16 * h),
+                                  r16);
                     }
+                }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bar_table));
             }
-            img_prev = img;
+            d_prev = d;
+            d = d_next;
         }
     } else if (warp == kTcMmaWarp) {
         // ---------------- MMA issuer ----------------
@@ -459,10 +506,11 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
             int cur_d = -1;
             uint32_t nchg = 0;
             int64_t issued = 0;
+            int d_next = tile_d[i0];
             for (int64_t k = 0; k < ntile && !*abort; ++k) {
-                const int64_t it = i0 + k;
                 const int st = (int)(k & 1);
-                const int d = tile_d[it];
+                const int d = d_next;
+                if (k + 1 < ntile) d_next = tile_d[i0 + k + 1];
                 bool ok = true;
                 if (d != cur_d) {
                     ok = mbar_wait_bounded(smem_u32(&bar_table), nchg & 1, kTcWait, abort);
@@ -504,12 +552,18 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
     } else if (warp < 8) {
         // ---------------- epilogue ----------------
         const int q = warp & 3, g = warp >> 2;  // lane quarter, column group (16-column chunks g, g + 2, ...)
+        int64_t p0n = tile_begin[i0];
+        int nn = tile_count[i0], dn = S::H == 2 ? tile_d[i0] : 0;
         for (int64_t k = 0; k < ntile && !warp_aborted(); ++k) {
-            const int64_t it = i0 + k;
             const int st = (int)(k & 1);
-            const int64_t p0 = tile_begin[it];
-            const int ncol = tile_count[it] * m;
-            const int h = S::H == 2 ? (tile_d[it] & 1) : 0;  // slot half of this pass
+            const int64_t p0 = p0n;
+            const int ncol = nn * m;
+            const int h = S::H == 2 ? (dn & 1) : 0;          // slot half of this pass
+            if (k + 1 < ntile) {
+                p0n = tile_begin[i0 + k + 1];
+                nn = tile_count[i0 + k + 1];
+                if (S::H == 2) dn = tile_d[i0 + k + 1];
+            }
             const int n = 128 * h + 32 * q + lane;            // output slot of this lane
             if (!warp_wait(&bar_accf[st], (uint32_t)((k >> 1) & 1))) {
                 if (lane == 0) give_up();
@@ -541,6 +595,25 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
         asm volatile("tcgen05.fence::after_thread_sync;");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TMEM_COLS));
     }
+}
+
+// Host: the tile ranges of G CTAs (G + 1 offsets) over a list of tiles with table indexes d, of
+// about equal cost: a tile one, a change of table kTcSwitch more.  A change drains the MMA, reads
+// 2 x 128 x KP words and writes them to tensor memory, which takes about three tiles' time: with
+// equal tile counts the CTAs holding the short runs of the upper levels (the Helmholtz form's
+// tables differ by level: hundreds of runs of one tile) ran three times as long as the others.
+constexpr int kTcSwitch = 3;
+inline std::vector<int64_t> tc_tile_ranges(const std::vector<int32_t>& d, int64_t G) {
+    const int64_t n = (int64_t)d.size();
+    std::vector<int64_t> r(G + 1, n);
+    int64_t total = 0;
+    for (int64_t i = 0; i < n; ++i) total += 1 + (i == 0 || d[i] != d[i - 1] ? kTcSwitch : 0);
+    int64_t cost = 0, g = 0;
+    for (int64_t i = 0; i < n; ++i) {
+        while (g < G && cost >= total * g / G) r[g++] = i;
+        cost += 1 + (i == 0 || d[i] != d[i - 1] ? kTcSwitch : 0);
+    }
+    return r;
 }
 
 // the autotuner's alternative tile of the real M2L: 80 columns where the default has 96
