@@ -155,13 +155,6 @@ struct Evaluator final : EvaluatorBase {
     ClosePairs close{};
     int64_t nclose = 0;
     static constexpr bool kMixed = sizeof(T) == 4;
-    // register P2M (f32, vectors one after another) up to p = 10; above, its (p+1)^2
-    // accumulators a lane exceed the register file (255 registers at p = 11, 12) and the
-    // shared-memory column sums run instead (p = 11, sphere 1e6: 0.19 against 0.24 ms).
-    // P2L keeps the register kernel at every order: its boxes sum many more sources, and
-    // the shared-memory form measured slower there (p = 11: 0.60 against 0.28 ms)
-    static constexpr bool kBfly = sizeof(T) == 4 && P <= 10;
-    static constexpr bool kBflyP2L = sizeof(T) == 4;
 
     // near-singular threshold of the mixed form: r2 < 1/16 in target-leaf units (|d| < r_t/4)
     static constexpr float kTheta2 = 0.0625f;
@@ -288,7 +281,7 @@ struct Evaluator final : EvaluatorBase {
             xbox_start[pl.nlevels] = (int64_t)xb.size();
             xbox.upload(xb);
             if (!xb.empty()) Lx.alloc(sizeof(T) * (size_t)m * ms_of(P) * pl.nboxes());
-            if (kMixed && !xb.empty()) {  // the f32 P2L's entry records
+            if (kBfly && !xb.empty()) {  // the register P2L's entry records
                 xrec.alloc(sizeof(XRec) * (pl.x.nnz() + 1));
                 x_record_kernel<<<(unsigned)((xb.size() + 127) / 128), 128>>>(dp, xbox.as<int32_t>(),
                                                                               (int64_t)xb.size(), xrec.as<XRec>());
@@ -320,11 +313,7 @@ struct Evaluator final : EvaluatorBase {
         close_pairs = nclose;
         gemm_setup<false>();
         // shared memory opt-in beyond 48 KB where a kernel needs it
-        size_t exp_smem = sizeof(T) * (NC * 32 + (size_t)m * 32);
-        if (exp_smem > 48 * 1024) {
-            CUDA_TRY(cudaFuncSetAttribute(expand_kernel<P, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)exp_smem));
-            CUDA_TRY(cudaFuncSetAttribute(expand_kernel<P, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)exp_smem));
-        }
+        static_assert(expand_smem<P, T>(kExpandMost) <= 47 * 1024, "P2M / P2L stage");
     }
 
     // The translation products Y[pair] = A_d X[source] of a tile list: f64 on the FP64 tensor
@@ -1278,22 +1267,35 @@ struct Evaluator final : EvaluatorBase {
                 d_charges, src_perm.as<int64_t>(), ns, m, qstride, sq.as<T>(), kMixed ? sq64.as<double>() : nullptr);
     }
 
-    size_t exp_smem() const { return sizeof(T) * (NC * 32 + (size_t)m * 32); }
-
-    void p2m_rows(int64_t r0, int64_t r1) {  // P2M of leaves [r0, r1)
-        if (r1 <= r0) return;
-        if (kBfly && m == 1)
-            expand_bfly_kernel<P, false, false><<<counted((unsigned)(r1 - r0)), 32, 0, stream>>>(
-                dp, r0, r1, nullptr, reinterpret_cast<const float4*>(spos.ptr), m,
-                reinterpret_cast<const float*>(sq.ptr), reinterpret_cast<float*>(M.ptr));
-        else if (kBfly)
-            expand_bfly_kernel<P, false, true><<<counted((unsigned)(r1 - r0)), 32, 0, stream>>>(
-                dp, r0, r1, nullptr, reinterpret_cast<const float4*>(spos.ptr), m,
-                reinterpret_cast<const float*>(sq.ptr), reinterpret_cast<float*>(M.ptr));
-        else
-            expand_kernel<P, T, false><<<counted((unsigned)(r1 - r0)), 32, exp_smem(), stream>>>(
-                dp, r0, r1, nullptr, m, spos.as<T4>(), sq.as<T>(), M.as<T>());
+    // P2M / P2L launches: the register form for a handle of one f32 vector (expand_bfly_kernel),
+    // else by the charge vectors a pass over the sources takes.  (The form goes by the handle's
+    // vectors, not the pass's, so the results do not depend on the vectors per pass.)
+    template <bool IRREG, int VB>
+    void expand(int64_t r0, int64_t r1, const int32_t* rows, T* out, cudaStream_t s) {
+        expand_kernel<P, T, IRREG, VB><<<counted((unsigned)(r1 - r0)), 32, expand_smem<P, T>(VB), s>>>(
+            dp, r0, r1, rows, m, spos.as<T4>(), sq.as<T>(), out);
     }
+    static constexpr int kExpandMost = kMixed ? 16 : 4;
+    static constexpr bool kBfly = kMixed && P <= 10;
+    template <bool IRREG>
+    void expand_vectors(int64_t r0, int64_t r1, const int32_t* rows, T* out, cudaStream_t s) {
+        if (r1 <= r0) return;
+        if constexpr (kBfly)
+            if (qstride == 1) {
+                expand_bfly_kernel<P, IRREG><<<counted((unsigned)(r1 - r0)), 32, 0, s>>>(
+                    dp, r0, r1, rows, reinterpret_cast<const float4*>(spos.ptr),
+                    reinterpret_cast<const float*>(sq.ptr), reinterpret_cast<float*>(out), xrec.as<XRec>());
+                return;
+            }
+        if (m == 1)
+            expand<IRREG, 1>(r0, r1, rows, out, s);
+        else if (m <= 4 || !kMixed)
+            expand<IRREG, 4>(r0, r1, rows, out, s);
+        else
+            expand<IRREG, kExpandMost>(r0, r1, rows, out, s);
+    }
+
+    void p2m_rows(int64_t r0, int64_t r1) { expand_vectors<false>(r0, r1, nullptr, M.as<T>(), stream); }
 
     template <bool CPLX = false>
     void m2m_level(int l, const T* tab, T* yo, T* mm) {  // parents on level l from their children on level l + 1
@@ -1367,19 +1369,7 @@ struct Evaluator final : EvaluatorBase {
 
     // P2L sums of the boxes [b0, b1) of the X box list into Lx, on stream s
     void p2l_rows(int64_t b0, int64_t b1, cudaStream_t s) {
-        if (b1 <= b0) return;
-        auto* out = reinterpret_cast<float*>(Lx.ptr);
-        if (kBflyP2L && m == 1)
-            expand_bfly_kernel<P, true, false><<<counted((unsigned)(b1 - b0)), 32, 0, s>>>(
-                dp, b0, b1, xbox.as<int32_t>(), reinterpret_cast<const float4*>(spos.ptr), m,
-                reinterpret_cast<const float*>(sq.ptr), out, xrec.as<XRec>());
-        else if (kBflyP2L)
-            expand_bfly_kernel<P, true, true><<<counted((unsigned)(b1 - b0)), 32, 0, s>>>(
-                dp, b0, b1, xbox.as<int32_t>(), reinterpret_cast<const float4*>(spos.ptr), m,
-                reinterpret_cast<const float*>(sq.ptr), out, xrec.as<XRec>());
-        else
-            expand_kernel<P, T, true><<<counted((unsigned)(b1 - b0)), 32, exp_smem(), s>>>(
-                dp, b0, b1, xbox.as<int32_t>(), m, spos.as<T4>(), sq.as<T>(), Lx.as<T>());
+        expand_vectors<true>(b0, b1, xbox.as<int32_t>(), Lx.as<T>(), s);
     }
 
     void leaf_far(int64_t r0, int64_t r1, int mode) {  // L2P / M2P of leaves [r0, r1)

@@ -95,93 +95,160 @@ __global__ void charge_load_kernel(const double* __restrict__ q_caller, const in
 }
 
 // ---------------------------------------------------------------------------------
-// P2M (rows = leaves, source = the leaf itself, unit frame) and P2L (rows = boxes,
-// sources = X-list leaves, frame (c(t|s), r(t|s))): one warp per row.  Each lane forms
-// the harmonics of one source and writes conj(X) into shared memory; lanes then sum
-// the 32 sources of a chunk per coefficient in source order.
+// P2M (rows = leaves, the leaf's own sources, unit frame) and P2L (rows = boxes, the sources
+// of the X-list leaves, frame (c(t|s), r(t|s))): one warp per row.
 //   multipole: M_n^m = sum q conj R_n^m(u);  X sum: X_n^m = sum q conj I_n^m((u - c)/r)
 // P2L writes its sums to an array of their own (Lx, a box's rows as in Lc), so that every
 // level's P2L is one launch beside the upward pass; the downward pass adds them.
+//
+// The row's sources, taken as one run over its entries, go 32 at a time: each lane forms one
+// source's harmonics (conj X, the slots of harmonics.cuh) into shared memory, then the lanes
+// hold the slots lane, lane + 32, ... and add q S over the 32 sources in order, for VB charge
+// vectors at a time, in registers.  The harmonics are so formed once per source and VB
+// vectors, and a run over the X entries fills the lanes where single leaves of 8 to 24 sources
+// left most of them idle: a batch of 700,000 points with 16 vectors at p = 6 takes 0.09 ms for
+// P2M and 0.44 for P2L, against 0.40 and 1.50 with the harmonics formed again for each vector
+// (in f64, whose shared-memory rows of 32 fell in one bank, P2M of 1e6 points at p = 8 takes
+// 0.08 ms against 0.20).  A vector's sums are the same floats for any VB.
+// A handle of one f32 vector keeps the register form below where it is the faster one.
 // ---------------------------------------------------------------------------------
-template <int P, typename T, bool IRREG>
+template <int P, typename T>
+constexpr int expand_smem(int vb) {
+    return (int)sizeof(T) * ((nc_of(P) * 33 + 3) / 4 * 4 + 32 * vb);
+}
+template <int P, typename T, bool IRREG, int VB>
 __global__ void __launch_bounds__(32) expand_kernel(DevPlan plan, int64_t row_begin, int64_t row_end,
                                                     const int32_t* __restrict__ rows, int m,
                                                     const typename Vec4<T>::type* __restrict__ spos,
                                                     const T* __restrict__ sq, T* __restrict__ out) {
-    constexpr int NC = nc_of(P);
-    extern __shared__ unsigned char smem_raw[];
-    T* S = reinterpret_cast<T*>(smem_raw);  // [NC][32]
-    T* Q = S + NC * 32;                     // [m][32]
+    using T4 = typename Vec4<T>::type;
+    using T2 = typename Pair2<T>::type;
+    constexpr int NC = nc_of(P), NCL = (NC + 31) / 32, SR = 33;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* S = reinterpret_cast<T*>(smem_raw);    // [NC][33]
+    T* Q = S + (NC * SR + 3) / 4 * 4;         // [32][VB]
+    __shared__ T4 ent_frame[IRREG ? 32 : 1];  // an entry's frame c and 1 / r
+    __shared__ int64_t ent_s0[IRREG ? 32 : 1];
+    __shared__ int ent_pre[IRREG ? 33 : 1];   // sources before it in the batch
     const int lane = threadIdx.x;
     const int64_t idx = row_begin + blockIdx.x;  // rows[idx] when a row list is given
     if (idx >= row_end) return;
     const int64_t row = rows ? rows[idx] : idx;
-    int box, nent;
-    int64_t ent0;
-    if (!IRREG) {  // row = leaf
-        box = plan.leaf_box[row];
-        nent = 1;
-        ent0 = 0;
-        if (plan.src_below[box] == 0) return;
-    } else {  // row = box
-        box = (int)row;
-        ent0 = plan.x_row[row];
-        nent = (int)(plan.x_row[row + 1] - ent0);
-        if (nent == 0) return;
-    }
-    T* outb = out + (int64_t)box * m * ms_of(P);
-    bool first = true;
-    for (int e = 0; e < nent; ++e) {
-        int sleaf = IRREG ? plan.x_col[ent0 + e] : (int)row;
-        T fc[3] = {T(0), T(0), T(0)};
-        T fr = T(1);
-        if (IRREG) rel_frame<T>(plan, box, plan.leaf_box[sleaf], fc, fr);  // (c(t|s), r(t|s))
-        T finv = T(1) / fr;
-        int64_t s0 = plan.src_start[sleaf], s1 = plan.src_start[sleaf + 1];
-        for (int64_t cb = s0; cb < s1; cb += 32) {
-            int64_t si = cb + lane;
-            bool valid = si < s1;
-            T x = T(0), y = T(0), z = T(1);
-            if (valid) {
-                auto p4 = spos[si];
-                x = (p4.x - fc[0]) * finv;
-                y = (p4.y - fc[1]) * finv;
-                z = (p4.z - fc[2]) * finv;
+    const int box = IRREG ? (int)row : plan.leaf_box[row];
+    const int64_t x0 = IRREG ? plan.x_row[row] : 0, x1 = IRREG ? plan.x_row[row + 1] : 1;
+    // a leaf without sources keeps its zero multipole
+    if (IRREG ? x0 == x1 : plan.src_start[row + 1] == plan.src_start[row]) return;
+    for (int v0 = 0; v0 < m; v0 += VB) {
+        const int nb = m - v0 < VB ? m - v0 : VB;
+        T2 acc[NCL][(VB + 1) / 2];
+#pragma unroll
+        for (int c = 0; c < NCL; ++c)
+#pragma unroll
+            for (int b = 0; b < (VB + 1) / 2; ++b) acc[c][b] = mk2(T(0), T(0));
+        for (int64_t e0 = x0; e0 < x1; e0 += 32) {
+            const int ne = x1 - e0 < 32 ? (int)(x1 - e0) : 32;
+            int64_t first = 0;  // P2M: the leaf's first source
+            int tot;
+            if constexpr (IRREG) {
+                __syncwarp();
+                int cnt = 0;
+                if (lane < ne) {
+                    const int sl = plan.x_col[e0 + lane];
+                    T c[3], r;
+                    rel_frame<T>(plan, box, plan.leaf_box[sl], c, r);  // (c(t|s), r(t|s))
+                    T4 f;
+                    f.x = c[0];
+                    f.y = c[1];
+                    f.z = c[2];
+                    f.w = T(1) / r;
+                    ent_frame[lane] = f;
+                    const int64_t s0 = plan.src_start[sl];
+                    ent_s0[lane] = s0;
+                    cnt = (int)(plan.src_start[sl + 1] - s0);
+                }
+                int sum = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= o) sum += y;
+                }
+                ent_pre[lane] = sum - cnt;
+                tot = __shfl_sync(0xffffffffu, sum, 31);
+                __syncwarp();
+            } else {
+                first = plan.src_start[row];
+                tot = (int)(plan.src_start[row + 1] - first);
             }
-            for (int v = 0; v < m; ++v) Q[v * 32 + lane] = valid ? sq[(int64_t)v * plan.nsrc + si] : T(0);
-            auto rows = [&](auto& h) {  // (pair rows, leaf_far_x2.cuh)
+            for (int cb = 0; cb < tot; cb += 32) {
+                const int pos = cb + lane;
+                if (pos < tot) {
+                    int64_t si = first + pos;
+                    T4 f;
+                    if constexpr (IRREG) {
+                        int lo = 0;  // the last entry starting at or before pos
 #pragma unroll
-                for (int n = 0; n <= P; ++n) {
-                    h.step(n);
+                        for (int b = 16; b; b >>= 1)
+                            if (lo + b < ne && ent_pre[lo + b] <= pos) lo += b;
+                        f = ent_frame[lo];
+                        si = ent_s0[lo] + (pos - ent_pre[lo]);
+                    }
+                    const T4 p4 = spos[si];
 #pragma unroll
-                    for (int mm = 0; mm <= n; ++mm) {
-                        S[slot(n, mm) * 32 + lane] = valid ? h.c[mm].x : T(0);
-                        if (mm) S[slot(n, -mm) * 32 + lane] = valid ? -h.c[mm].y : T(0);
+                    for (int b = 0; b < VB; ++b)
+                        Q[lane * VB + b] = b < nb ? sq[(int64_t)(v0 + b) * plan.nsrc + si] : T(0);
+                    auto slots = [&](auto& h) {
+#pragma unroll
+                        for (int n = 0; n <= P; ++n) {
+                            h.step(n);
+#pragma unroll
+                            for (int mm = 0; mm <= n; ++mm) {
+                                S[slot(n, mm) * SR + lane] = h.c[mm].x;
+                                if (mm) S[slot(n, -mm) * SR + lane] = -h.c[mm].y;
+                            }
+                        }
+                    };
+                    if constexpr (IRREG) {
+                        const T x = (p4.x - f.x) * f.w, y = (p4.y - f.y) * f.w, z = (p4.z - f.z) * f.w;
+                        IrregularRows2<P, T> h;
+                        h.init(x, y, z, T(1) / sqrt(x * x + y * y + z * z));
+                        slots(h);
+                    } else {
+                        RegularRows2<P, T> h;
+                        h.init(p4.x, p4.y, p4.z);
+                        slots(h);
                     }
                 }
-            };
-            if constexpr (!IRREG) {
-                RegularRows2<P, T> h;
-                h.init(x, y, z);
-                rows(h);
-            } else {
-                IrregularRows2<P, T> h;
-                const T r2 = x * x + y * y + z * z;
-                h.init(x, y, z, valid ? T(1) / sqrt(r2) : T(0));
-                rows(h);
-            }
-            __syncwarp();
-            int cnt = (int)((s1 - cb) < 32 ? (s1 - cb) : 32);
-            for (int v = 0; v < m; ++v)
-                for (int c = lane; c < NC; c += 32) {
-                    T acc = T(0);
-                    for (int j = 0; j < cnt; ++j) acc += Q[v * 32 + j] * S[c * 32 + j];
-                    T* o = outb + (int64_t)v * ms_of(P) + c;
-                    if (first) *o = acc;
-                    else *o += acc;
+                __syncwarp();
+                const int cnt = tot - cb < 32 ? tot - cb : 32;
+#pragma unroll 2
+                for (int j = 0; j < cnt; ++j) {
+                    T s[NCL];
+#pragma unroll
+                    for (int c = 0; c < NCL; ++c) s[c] = S[(lane + 32 * c < NC ? lane + 32 * c : 0) * SR + j];
+                    if constexpr (VB == 1) {
+                        const T q = Q[j];
+#pragma unroll
+                        for (int c = 0; c < NCL; ++c) acc[c][0].x = fma1(q, s[c], acc[c][0].x);
+                    } else {
+                        const T2* q2 = reinterpret_cast<const T2*>(Q + j * VB);
+#pragma unroll
+                        for (int b = 0; b < VB / 2; ++b) {
+                            const T2 q = q2[b];
+#pragma unroll
+                            for (int c = 0; c < NCL; ++c) acc[c][b] = fma2(q, x2(s[c]), acc[c][b]);
+                        }
+                    }
                 }
-            first = false;
-            __syncwarp();
+                __syncwarp();
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NCL; ++c) {
+            const int k = lane + 32 * c;
+            if (k >= NC) break;
+#pragma unroll
+            for (int b = 0; b < VB; ++b)
+                if (b < nb) out[((int64_t)box * m + v0 + b) * ms_of(P) + k] = b & 1 ? acc[c][b / 2].y : acc[c][b / 2].x;
         }
     }
 }
@@ -191,7 +258,10 @@ __global__ void __launch_bounds__(32) expand_kernel(DevPlan plan, int64_t row_be
 // j, j+32, ... of every entry and accumulates q conj(X) for all (p+1)^2 slots in
 // registers; one butterfly reduce-scatter per row then leaves every lane with
 // NCP/32 finished slots (NCP = slots padded to a multiple of 32).  The summation order
-// is fixed (per-lane partial sums, then a fixed tree), so results are repeatable.
+// is fixed (per-lane partial sums, then a fixed tree), so results are repeatable.  It serves
+// handles of one vector: P2M to p = 10 (above, its (p+1)^2 sums exceed the register file: 0.19
+// against 0.08 ms for 1e6 points at p = 11) and P2L to p = 10 (4e6 points of a sphere at p = 8
+// 0.22 against 0.31 ms; at p = 11 0.20 against 0.16).
 // ---------------------------------------------------------------------------------
 // One X-list entry of the f32 P2L, fixed at build (x_record_kernel): the source leaf's
 // frame seen from the target box, (c(t|s), r(t|s)) of rel_frame<float>, and its sources,
@@ -222,10 +292,10 @@ static __global__ void x_record_kernel(DevPlan plan, const int32_t* __restrict__
     }
 }
 
-template <int P, bool IRREG, bool MULTI>
+template <int P, bool IRREG>
 __global__ void __launch_bounds__(32) expand_bfly_kernel(DevPlan plan, int64_t row_begin, int64_t row_end,
                                                          const int32_t* __restrict__ rows,
-                                                         const float4* __restrict__ spos, int m,
+                                                         const float4* __restrict__ spos,
                                                          const float* __restrict__ sq, float* __restrict__ out,
                                                          const XRec* __restrict__ xrec = nullptr) {
     constexpr int NC = nc_of(P);
@@ -249,10 +319,6 @@ __global__ void __launch_bounds__(32) expand_bfly_kernel(DevPlan plan, int64_t r
         nent = (int)(plan.x_row[row + 1] - ent0);
         if (nent == 0) return;
     }
-    // the charge vectors one after the other (charges [v][point], expansions [box][v]);
-    // MULTI = false compiles the one-vector form (m = 1) without the loop's registers
-    for (int v = 0; v < (MULTI ? m : 1); ++v) {
-    const float* qv = sq + (int64_t)v * plan.nsrc;
     float w[NCP];
 #pragma unroll
     for (int c = 0; c < NCP; ++c) w[c] = 0.0f;
@@ -282,14 +348,14 @@ __global__ void __launch_bounds__(32) expand_bfly_kernel(DevPlan plan, int64_t r
         float qn = 0.f;
         if (si < s1) {
             pn = spos[si];
-            qn = qv[si];
+            qn = sq[si];
         }
         for (; si < s1; si += 32) {
             const float4 p4 = pn;
             const float q = qn;
             if (si + 32 < s1) {
                 pn = spos[si + 32];
-                qn = qv[si + 32];
+                qn = sq[si + 32];
             }
             const float x = (p4.x - fc[0]) * finv, y = (p4.y - fc[1]) * finv, z = (p4.z - fc[2]) * finv;
             // conj(X) q into the slots: (w[slot(n, mm)], w[slot(n, -mm)]) += (q, -q) * X_n^mm,
@@ -343,12 +409,11 @@ __global__ void __launch_bounds__(32) expand_bfly_kernel(DevPlan plan, int64_t r
 #pragma unroll
     for (int s = 16, len = NCP / 2; s >= 1; s >>= 1, len >>= 1)
         if (lane & s) base += len;
-    float* o = out + ((int64_t)box * m + v) * ms_of(P);
+    float* o = out + (int64_t)box * ms_of(P);
 #pragma unroll
     for (int i = 0; i < NCP / 32; ++i) {
         const int c = base + i;
         if (c < NC) o[c] = w[i];
-    }
     }
 }
 
