@@ -473,6 +473,7 @@ void build_device(fmmgpu_fmm* f, const std::vector<double>& us, const std::vecto
                              mixed && f->fused, f->ybudget};
     f->eval = make_evaluator(s.p, mixed, args, &bytes);
     f->eval->qstride = s.vectors;
+    f->eval->near_pairs = f->near_pairs;
     const size_t ns = P.src_perm.size(), nt = P.tgt_perm.size();
     f->d_charges.alloc(sizeof(double) * (size_t)s.vectors * (ns + 1));
     f->d_phi.alloc(sizeof(double) * (size_t)s.vectors * (nt + 1));

@@ -127,7 +127,13 @@ struct EvaluatorBase {
     int64_t launches = 0;  // kernels launched by the last evaluation
     int qstride = 1;       // charges per point in the caller's array (all vectors)
     bool first_pass = true;  // vectors run in passes: the first one resets timing and counts
-    bool overlap = false;  // near field on its own stream beside the far field (measured: no gain)
+    bool overlap = false;  // near field on its own stream beside the far field, whatever its size
+    int64_t near_pairs = 0;  // of the plan
+    // The near field of at most this many pairs and vectors runs beside the far field without
+    // being asked: it leaves SMs idle and so does the far field's chain of levels.  Above, both
+    // fill the device and sharing it costs more than it hides (measured beside each other: 30,011
+    // points, 16 M pairs, 199 against 181 us; a cube of 1e5 points in f64, 58 M, 310 against 289).
+    static constexpr int64_t kApartPairs = 200000000;
     // launch shapes the autotuner may change: warps a block of the mixed P2P kernel
     // (1, 2 or 4) and threads a block of the L2P / M2P kernel (32, 64 or 128)
     int p2p_warps = 4;  // the static block, kX2Warps of p2p_x2.cuh (checked there)
