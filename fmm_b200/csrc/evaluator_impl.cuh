@@ -1542,8 +1542,9 @@ struct Evaluator final : EvaluatorBase {
                 hq.alloc(sizeof(Cplx<T>) * (size_t)m * (dp.nsrc + 1));
                 if (kMixed) hq64.alloc(sizeof(double2) * (size_t)m * (dp.nsrc + 1));
             }
-            size_t smem = sizeof(double) * (2 * NC * 32 + 2 * (size_t)m * 32);
-            if (smem > 227 * 1024) throw Failure(FMMGPU_UNSUPPORTED, "too many charge vectors a pass for P2L");
+            const size_t smem = hh_expand_smem<P>(true, m);
+            if (sizeof(double) * 64 * (NC + (size_t)m) > 227 * 1024)
+                throw Failure(FMMGPU_UNSUPPORTED, "too many charge vectors a pass for P2L");
             CUDA_TRY(cudaFuncSetAttribute(hh_expand_kernel<P, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
             CUDA_TRY(cudaFuncSetAttribute(hh_expand_kernel<P, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1686,19 +1687,18 @@ struct Evaluator final : EvaluatorBase {
                 d_q, src_perm.as<int64_t>(), ns, m, qstride, hq.as<Cplx<T>>(), kMixed ? hq64.as<double2>() : nullptr);
         const int64_t top = plan.nlevels > 2 ? plan.level_start[2] : (int64_t)plan.nboxes();
         CUDA_TRY(cudaMemsetAsync(hh.L.ptr, 0, sizeof(T) * (size_t)mv * ms_of(P) * top, stream));
-        const size_t esmem = sizeof(double) * (2 * NC * 32 + 2 * (size_t)m * 32);
         // beside the upward pass: the P2L of every level, into hh.Lx
         const int64_t nx = xbox_start[plan.nlevels];
         if (nx) {
             CUDA_TRY(cudaEventRecord(ev_fork, stream));
             CUDA_TRY(cudaStreamWaitEvent(near_stream, ev_fork, 0));
-            hh_expand_kernel<P, T, true><<<counted((unsigned)nx), 32, esmem, near_stream>>>(
+            hh_expand_kernel<P, T, true><<<counted((unsigned)nx), 32, hh_expand_smem<P>(true, m), near_stream>>>(
                 dp, hh.lv, 0, nx, xbox.as<int32_t>(), m, spos.as<T4>(), hq.as<Cplx<T>>(), hh.Lx.as<T>());
             CUDA_TRY(cudaEventRecord(ev_x, near_stream));
         }
         // upward: P2M of every leaf, then M2M from level L-1 up to 0
         if (plan.nleaves())
-            hh_expand_kernel<P, T, false><<<counted((unsigned)plan.nleaves()), 32, esmem, stream>>>(
+            hh_expand_kernel<P, T, false><<<counted((unsigned)plan.nleaves()), 32, hh_expand_smem<P>(false, m), stream>>>(
                 dp, hh.lv, 0, (int64_t)plan.nleaves(), nullptr, m, spos.as<T4>(), hq.as<Cplx<T>>(), hM);
         upward<true>(hh.m2m.as<T>(), (int64_t)(8 * set), hh.Yo.as<T>(), hM);
         // M2L products of every level (their tables are per level): the mixed form on the

@@ -274,6 +274,14 @@ struct HhLevels {
 // for P2L), then the lanes add q B over the chunk's 32 sources per coefficient in source
 // order, into rows 2v (real) and 2v + 1 (imaginary) of the box's expansion.
 // ---------------------------------------------------------------------------------
+// (rows of 33: with 32 the lanes' slots of one source fell in one bank)
+constexpr int kHhBaseRow = 33;
+constexpr int kHhVectors = 64;  // charge vectors whose charges are staged at once
+template <int P>
+constexpr size_t hh_expand_smem(bool singular, int m) {
+    return sizeof(double) *
+           ((singular ? 2 : 1) * nc_of(P) * kHhBaseRow + 2 * (size_t)(m < kHhVectors ? m : kHhVectors) * 32);
+}
 template <int P, typename T, bool SINGULAR>
 __global__ void __launch_bounds__(32) hh_expand_kernel(DevPlan plan, HhLevels lv, int64_t row_begin, int64_t row_end,
                                                        const int32_t* __restrict__ rows, int m,
@@ -281,9 +289,10 @@ __global__ void __launch_bounds__(32) hh_expand_kernel(DevPlan plan, HhLevels lv
                                                        const Cplx<T>* __restrict__ sq, T* __restrict__ out) {
     constexpr int NC = nc_of(P), MS = ms_of(P);
     constexpr int NB = SINGULAR ? 2 * NC : NC;  // real base (P2M) or complex base (P2L)
+    constexpr int BR = kHhBaseRow;
     extern __shared__ unsigned char smem_raw[];
-    double* B = reinterpret_cast<double*>(smem_raw);  // [NB][32]
-    double* Q = B + NB * 32;                          // [m][2][32]
+    double* B = reinterpret_cast<double*>(smem_raw);  // [NB][BR]
+    double* Q = B + NB * BR;                          // [m][2][32]
     const int lane = threadIdx.x;
     const int64_t idx = row_begin + blockIdx.x;
     if (idx >= row_end) return;
@@ -304,6 +313,8 @@ __global__ void __launch_bounds__(32) hh_expand_kernel(DevPlan plan, HhLevels lv
     const double kl = lv.kl[plan.level[box]], s = hh_scale(kl);
     const double pik = 4.0 * 3.14159265358979323846 * kl;
     T* outb = out + (int64_t)box * 2 * m * MS;
+    for (int v0 = 0; v0 < m; v0 += kHhVectors) {
+    const int nv = m - v0 < kHhVectors ? m - v0 : kHhVectors;
     bool first = true;  // the row's sums start from its first 32 sources
     for (int e = 0; e < nent; ++e) {
         const int sleaf = SINGULAR ? plan.x_col[ent0 + e] : (int)row;
@@ -321,8 +332,8 @@ __global__ void __launch_bounds__(32) hh_expand_kernel(DevPlan plan, HhLevels lv
                 y = ((double)p4.y - fc[1]) * finv;
                 z = ((double)p4.z - fc[2]) * finv;
             }
-            for (int v = 0; v < m; ++v) {
-                const Cplx<T> q = valid ? sq[(int64_t)v * plan.nsrc + si] : Cplx<T>{T(0), T(0)};
+            for (int v = 0; v < nv; ++v) {
+                const Cplx<T> q = valid ? sq[(int64_t)(v0 + v) * plan.nsrc + si] : Cplx<T>{T(0), T(0)};
                 Q[(2 * v) * 32 + lane] = (double)q.re;
                 Q[(2 * v + 1) * 32 + lane] = (double)q.im;
             }
@@ -333,40 +344,40 @@ __global__ void __launch_bounds__(32) hh_expand_kernel(DevPlan plan, HhLevels lv
                 const int tp = n * n + n + mm, tn = n * n + n - mm;
                 if (!SINGULAR) {
                     const double w = valid ? rad.jh[n] : 0.0;
-                    B[tp * 32 + lane] = w * yc;
-                    if (mm) B[tn * 32 + lane] = w * ys;
+                    B[tp * BR + lane] = w * yc;
+                    if (mm) B[tn * BR + lane] = w * ys;
                 } else {
                     // 4 pi i k hh_n Y
                     const double wr = valid ? -pik * rad.hi[n] : 0.0, wi = valid ? pik * rad.hr[n] : 0.0;
-                    B[tp * 32 + lane] = wr * yc;
-                    B[(NC + tp) * 32 + lane] = wi * yc;
+                    B[tp * BR + lane] = wr * yc;
+                    B[(NC + tp) * BR + lane] = wi * yc;
                     if (mm) {
-                        B[tn * 32 + lane] = wr * ys;
-                        B[(NC + tn) * 32 + lane] = wi * ys;
+                        B[tn * BR + lane] = wr * ys;
+                        B[(NC + tn) * BR + lane] = wi * ys;
                     }
                 }
             });
             __syncwarp();
             const int cnt = (int)((s1 - cb) < 32 ? (s1 - cb) : 32);
-            for (int v = 0; v < m; ++v) {
+            for (int v = 0; v < nv; ++v) {
                 const double* qr = Q + (2 * v) * 32;
                 const double* qi = Q + (2 * v + 1) * 32;
                 for (int t = lane; t < NC; t += 32) {
                     double ar = 0.0, ai = 0.0;
                     if (!SINGULAR) {
                         for (int j = 0; j < cnt; ++j) {
-                            const double b = B[t * 32 + j];
+                            const double b = B[t * BR + j];
                             ar += qr[j] * b;
                             ai += qi[j] * b;
                         }
                     } else {
                         for (int j = 0; j < cnt; ++j) {
-                            const double br = B[t * 32 + j], bi = B[(NC + t) * 32 + j];
+                            const double br = B[t * BR + j], bi = B[(NC + t) * BR + j];
                             ar += qr[j] * br - qi[j] * bi;
                             ai += qr[j] * bi + qi[j] * br;
                         }
                     }
-                    T* o = outb + (int64_t)(2 * v) * MS + t;
+                    T* o = outb + (int64_t)(2 * (v0 + v)) * MS + t;
                     o[0] = first ? (T)ar : (T)((double)o[0] + ar);
                     o[MS] = first ? (T)ai : (T)((double)o[MS] + ai);
                 }
@@ -374,6 +385,7 @@ __global__ void __launch_bounds__(32) hh_expand_kernel(DevPlan plan, HhLevels lv
             first = false;
             __syncwarp();
         }
+    }
     }
 }
 
@@ -384,66 +396,52 @@ __global__ void __launch_bounds__(32) hh_expand_kernel(DevPlan plan, HhLevels lv
 template <int P, bool GRAD, bool SINGULAR, typename T>
 __device__ __forceinline__ void hh_eval(const T* __restrict__ E, double k, double s, double vx, double vy, double vz,
                                         double (&out)[8]) {
-    constexpr int NC = nc_of(P), MS = ms_of(P);
+    constexpr int MS = ms_of(P);
     const double d = sqrt(vx * vx + vy * vy + vz * vz);
     HhRadial<P, SINGULAR> rad;
     rad.eval(k * d, s, GRAD);
-    // per degree: S_n = sum_m E Y, and with GRAD T_n = sum_m E d_t Y, F_n = sum_m E d_f Y / sin t
-    double Sr[P + 1], Si[P + 1], Tr[P + 1], Ti[P + 1], Fr[P + 1], Fi[P + 1];
-#pragma unroll
-    for (int n = 0; n <= P; ++n) Sr[n] = Si[n] = Tr[n] = Ti[n] = Fr[n] = Fi[n] = 0.0;
+    // Each harmonic's terms go straight into the sums with its degree's radial factors: the
+    // value, the radial derivative (times k at the end) and the two angular derivatives
+    // (over |v| at the end).  Sums kept per degree until the end held 6 (P + 1) values a
+    // thread beside the harmonics' columns and, with every harmonic hoisted out of the vector
+    // loop, spilled 2.6 KB a thread at p = 10.
+    double f[2] = {0.0, 0.0}, gr[2] = {0.0, 0.0}, gt[2] = {0.0, 0.0}, gf[2] = {0.0, 0.0};
+    auto add = [&](double (&o)[2], double re, double im, double wr, double wi) {
+        o[0] = fma(re, wr, o[0]);
+        o[1] = fma(im, wr, o[1]);
+        if (SINGULAR) {
+            o[0] = fma(-im, wi, o[0]);
+            o[1] = fma(re, wi, o[1]);
+        }
+    };
     hh_harmonics<P, GRAD>(vx, vy, vz, [&](int n, int mm, double yc, double ys, double tc, double ts, double fc, double fs) {
         const int tp = n * n + n + mm, tn = n * n + n - mm;
         const double er = (double)E[tp], ei = (double)E[MS + tp];
-        Sr[n] += er * yc;
-        Si[n] += ei * yc;
-        if (GRAD) {
-            Tr[n] += er * tc;
-            Ti[n] += ei * tc;
-            Fr[n] += er * fc;
-            Fi[n] += ei * fc;
-        }
+        double Sr = er * yc, Si = ei * yc, Tr = er * tc, Ti = ei * tc, Fr = er * fc, Fi = ei * fc;
         if (mm) {
             const double nr = (double)E[tn], ni = (double)E[MS + tn];
-            Sr[n] += nr * ys;
-            Si[n] += ni * ys;
-            if (GRAD) {
-                Tr[n] += nr * ts;
-                Ti[n] += ni * ts;
-                Fr[n] += nr * fs;
-                Fi[n] += ni * fs;
-            }
+            Sr = fma(nr, ys, Sr);
+            Si = fma(ni, ys, Si);
+            Tr = fma(nr, ts, Tr);
+            Ti = fma(ni, ts, Ti);
+            Fr = fma(nr, fs, Fr);
+            Fi = fma(ni, fs, Fi);
+        }
+        const double wr = SINGULAR ? rad.hr[n] : rad.jh[n], wi = SINGULAR ? rad.hi[n] : 0.0;
+        add(f, Sr, Si, wr, wi);
+        if (GRAD) {
+            add(gr, Sr, Si, SINGULAR ? rad.hpr[n] : rad.jhp[n], SINGULAR ? rad.hpi[n] : 0.0);
+            add(gt, Tr, Ti, wr, wi);
+            add(gf, Fr, Fi, wr, wi);
         }
     });
-    (void)NC;
-    double f[2] = {0.0, 0.0}, gr[2] = {0.0, 0.0}, gt[2] = {0.0, 0.0}, gf[2] = {0.0, 0.0};
+    if (GRAD) {
+        const double id = d > 0.0 ? 1.0 / d : 0.0;
 #pragma unroll
-    for (int n = 0; n <= P; ++n) {
-        double Rr, Ri, Pr, Pi, Ur, Ui;  // value, k * derivative, value / |v|
-        if (SINGULAR) {
-            Rr = rad.hr[n];
-            Ri = rad.hi[n];
-            Pr = GRAD ? k * rad.hpr[n] : 0.0;
-            Pi = GRAD ? k * rad.hpi[n] : 0.0;
-            Ur = Rr / d;
-            Ui = Ri / d;
-        } else {
-            Rr = rad.jh[n];
-            Ri = 0.0;
-            Pr = k * rad.jhp[n];
-            Pi = 0.0;
-            Ur = d > 0.0 ? rad.jh[n] / d : (n == 1 ? k / (3.0 * s) : 0.0);
-            Ui = 0.0;
-        }
-        f[0] += Sr[n] * Rr - Si[n] * Ri;
-        f[1] += Sr[n] * Ri + Si[n] * Rr;
-        if (GRAD) {
-            gr[0] += Sr[n] * Pr - Si[n] * Pi;
-            gr[1] += Sr[n] * Pi + Si[n] * Pr;
-            gt[0] += Tr[n] * Ur - Ti[n] * Ui;
-            gt[1] += Tr[n] * Ui + Ti[n] * Ur;
-            gf[0] += Fr[n] * Ur - Fi[n] * Ui;
-            gf[1] += Fr[n] * Ui + Fi[n] * Ur;
+        for (int c = 0; c < 2; ++c) {
+            gr[c] *= k;
+            gt[c] *= id;
+            gf[c] *= id;
         }
     }
     out[0] = f[0];
@@ -500,8 +498,11 @@ __global__ void __launch_bounds__(128) hh_leaf_far_kernel(DevPlan plan, HhLevels
     const double kt = lv.kl[plan.level[box]], st = hh_scale(kt);
     for (int64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
         const auto p4 = tpos[t];
-        const double ux = (double)p4.x, uy = (double)p4.y, uz = (double)p4.z;
         for (int v = 0; v < m; ++v) {
+            // an opaque copy of the position each vector, or the harmonics are formed before the
+            // loop as its invariants, all of them live across it, and spilled
+            double ux = (double)p4.x, uy = (double)p4.y, uz = (double)p4.z;
+            asm volatile("" : "+d"(ux), "+d"(uy), "+d"(uz));
             double acc[8];
             hh_eval<P, GRAD, false, T>(Lc + ((int64_t)box * 2 * m + 2 * v) * MS, kt, st, ux, uy, uz, acc);
             for (int64_t e = w0; e < w1; ++e) {
