@@ -15,9 +15,9 @@
 // partials added in flush order all the same, so a target's sums are the same floats whatever
 // the number of items in the plan.
 //
-// Measured (gradients): 774.5 M near pairs of a cube of 1e6 points in 1.73 ms, 0.45 T pairs/s,
+// Measured (gradients): 774.5 M near pairs of a cube of 1e6 points in 1.49 ms, 0.52 T pairs/s,
 // against 2.04 ms for a lane a target with rsqrt(); whole evaluations, with the translations
-// unchanged: a cube of 2,500 points 82 -> 44 us (8 warps an item), of 1e6 5.96 -> 5.63 ms;
+// unchanged: a cube of 2,500 points 82 -> 44 us (8 warps an item), of 1e6 5.96 -> 5.39 ms;
 // Helmholtz on 40,009 points 1.30 -> 0.78 ms.
 //
 // The rules of the reference's device kernels hold: d = u_t - y, r2 by explicit fma, and a
@@ -161,9 +161,18 @@ constexpr int near_stage_doubles() {  // x, y, z, charges, in 16-byte pairs
     return (3 + PK::Q + 1) / 2 * 2;
 }
 
+// Blocks an SM of the warp-an-item form with one vector: five (20 warps, 102 registers), since
+// a pair's dependent chain and not the FP64 pipe bounds a warp: 1e6 points of a cube 1.49 ms
+// against 1.73 with the 154 registers and 12 warps the compiler takes unasked (six blocks 1.50;
+// two pairs in flight instead of four 1.58 to 1.61).
+template <class PK>
+constexpr int near_blocks(bool share) {
+    return share || PK::HELM || PK::VB > 1 ? 1 : 5;
+}
+
 // SHARE: the block's warps share one item (its flushes dealt round robin); else a warp an item.
 template <class PK, bool SHARE>
-__global__ void __launch_bounds__(SHARE ? 256 : 32 * kNearWarps) near_f64_kernel(NearArgs A) {
+__global__ void __launch_bounds__(SHARE ? 256 : 32 * kNearWarps, near_blocks<PK>(SHARE)) near_f64_kernel(NearArgs A) {
     constexpr int SD = near_stage_doubles<PK>(), C = PK::C;
     constexpr bool HELM = PK::HELM;
     constexpr int RW = SHARE ? 1 : kNearWarps;  // record sets a block
