@@ -450,8 +450,10 @@ class Fmm(Plan):
         f32 = np.asarray(charges).dtype == np.float32
         dt = np.float32 if f32 else np.float64
         q = np.ascontiguousarray(charges, dtype=dt).reshape(self.nsources, m)
-        phi = np.zeros((m, self.ntargets), dtype=dt)
-        g = np.zeros((m, self.ntargets, 3), dtype=dt) if self.settings.gradients else None
+        # every element is written by the call: not cleared first (16 MB of zeros cost 1.1 of a
+        # 4.7 ms call at 1e6 points)
+        phi = np.empty((m, self.ntargets), dtype=dt)
+        g = np.empty((m, self.ntargets, 3), dtype=dt) if self.settings.gradients else None
         call = lib().fmmgpu_fmm_evaluate_f32 if f32 else lib().fmmgpu_fmm_evaluate
         _check(call(self._h, _ptr(q), _ptr(phi), _ptr(g)))
         return Output(phi, g)
@@ -461,8 +463,8 @@ class Fmm(Plan):
         plan, complex charges (ns, m): Output with complex potential (m, nt) and gradient."""
         m = self.settings.vectors
         q = np.ascontiguousarray(charges, dtype=np.complex128).reshape(self.nsources, m)
-        phi = np.zeros((m, self.ntargets), dtype=np.complex128)
-        g = np.zeros((m, self.ntargets, 3), dtype=np.complex128) if self.settings.gradients else None
+        phi = np.empty((m, self.ntargets), dtype=np.complex128)
+        g = np.empty((m, self.ntargets, 3), dtype=np.complex128) if self.settings.gradients else None
         k = complex(k)
         _check(lib().fmmgpu_helmholtz_near(self._h, k.real, k.imag, _ptr(q), _ptr(phi), _ptr(g)))
         return Output(phi, g)
@@ -477,8 +479,8 @@ class Fmm(Plan):
         c64 = np.asarray(charges).dtype == np.complex64
         dt = np.complex64 if c64 else np.complex128
         q = np.ascontiguousarray(charges, dtype=dt).reshape(self.nsources, m)
-        phi = np.zeros((m, self.ntargets), dtype=dt)
-        g = np.zeros((m, self.ntargets, 3), dtype=dt) if self.settings.gradients else None
+        phi = np.empty((m, self.ntargets), dtype=dt)
+        g = np.empty((m, self.ntargets, 3), dtype=dt) if self.settings.gradients else None
         k = complex(k)
         call = lib().fmmgpu_helmholtz_evaluate_f32 if c64 else lib().fmmgpu_helmholtz_evaluate
         _check(call(self._h, k.real, k.imag, _ptr(q), _ptr(phi), _ptr(g)))
@@ -500,9 +502,9 @@ class Fmm(Plan):
         m = self.settings.vectors
         q = np.ascontiguousarray(charges, dtype=np.float64).reshape(self.nsources, m)
         w = np.ascontiguousarray(cotangent, dtype=np.float64).reshape(m, self.ntargets)
-        dq = np.zeros((self.nsources, m))
-        dxs = np.zeros((self.nsources, 3))
-        dxt = np.zeros((self.ntargets, 3))
+        dq = np.empty((self.nsources, m))
+        dxs = np.empty((self.nsources, 3))
+        dxt = np.empty((self.ntargets, 3))
         _check(lib().fmmgpu_fmm_vjp(self._h, _ptr(q), _ptr(w), _ptr(dq), _ptr(dxs), _ptr(dxt)))
         return dq, dxs, dxt
 
@@ -529,8 +531,8 @@ class Fmm(Plan):
                 calls += [("l2p", lv), ("m2p", lv), ("p2p", lv)]
         for kind, lv in calls:
             _check(getattr(L, "fmmgpu_op_" + kind)(self._h, lv))
-        phi = np.zeros((m, self.ntargets))
-        g = np.zeros((m, self.ntargets, 3)) if self.settings.gradients else None
+        phi = np.empty((m, self.ntargets))
+        g = np.empty((m, self.ntargets, 3)) if self.settings.gradients else None
         _check(L.fmmgpu_op_read_output(self._h, _ptr(phi), _ptr(g)))
         return Output(phi, g)
 

@@ -784,11 +784,13 @@ int fmmgpu_fmm_vjp(fmmgpu_fmm* f, const double* charges, const double* cotangent
             }
             T = f->transpose;
         }
-        f->d_vjp_w.alloc(sizeof(double) * (size_t)m * (nt + 1));
-        f->d_vjp_tq.alloc(sizeof(double) * (size_t)m * (nt + 1));
-        f->d_vjp_dq.alloc(sizeof(double) * (size_t)m * (ns + 1));
-        f->d_vjp_dxs.alloc(sizeof(double) * 3 * (ns + 1));
-        f->d_vjp_dxt.alloc(sizeof(double) * 3 * (nt + 1));
+        if (!f->d_vjp_dxt.ptr) {  // the handle's sizes do not change: kept for its later calls
+            f->d_vjp_w.alloc(sizeof(double) * (size_t)m * (nt + 1));
+            f->d_vjp_tq.alloc(sizeof(double) * (size_t)m * (nt + 1));
+            f->d_vjp_dq.alloc(sizeof(double) * (size_t)m * (ns + 1));
+            f->d_vjp_dxs.alloc(sizeof(double) * 3 * (ns + 1));
+            f->d_vjp_dxt.alloc(sizeof(double) * 3 * (nt + 1));
+        }
         cudaStream_t s = f->stream;
         CUDA_TRY(cudaMemcpyAsync(f->d_charges.ptr, charges, sizeof(double) * m * ns, cudaMemcpyHostToDevice, s));
         CUDA_TRY(cudaMemcpyAsync(f->d_vjp_w.ptr, cotangent, sizeof(double) * m * nt, cudaMemcpyHostToDevice, s));
