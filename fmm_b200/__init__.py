@@ -546,7 +546,8 @@ class Fmm(Plan):
         _check(lib().fmmgpu_fmm_set_kind_timing(self._h, int(on)))
 
     def set_overlap(self, on=True):
-        """Near field on a second stream beside the far field (default off)."""
+        """Near field on a second stream beside the far field (on), or after it (off); until it is
+        set the plan's size decides.  The same floats."""
         _check(lib().fmmgpu_fmm_set_overlap(self._h, int(on)))
 
     def set_graph(self, on=True):

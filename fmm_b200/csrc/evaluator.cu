@@ -1087,7 +1087,7 @@ int fmmgpu_fmm_set_overlap(fmmgpu_fmm* f, int on) {
         if (!f || !f->eval) throw Failure(FMMGPU_INVALID_ARGUMENT, "null argument or plan-only handle");
         CUDA_TRY(cudaSetDevice(f->settings.device));
         CUDA_TRY(cudaStreamSynchronize(f->stream));
-        f->eval->overlap = on != 0;
+        f->eval->overlap = on != 0 ? 1 : 0;
         f->drop_graph();
     });
 }

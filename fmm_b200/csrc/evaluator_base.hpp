@@ -127,10 +127,10 @@ struct EvaluatorBase {
     int64_t launches = 0;  // kernels launched by the last evaluation
     int qstride = 1;       // charges per point in the caller's array (all vectors)
     bool first_pass = true;  // vectors run in passes: the first one resets timing and counts
-    bool overlap = false;  // near field on its own stream beside the far field, whatever its size
+    // near field on its own stream beside the far field: 1 on, 0 off (set_overlap), -1 by size
+    int overlap = -1;
     int64_t near_pairs = 0;  // of the plan
-    // The near field of at most this many pairs and vectors runs beside the far field without
-    // being asked: it leaves SMs idle and so does the far field's chain of levels.  Above, both
+    // By size, the near field of at most this many pairs and vectors runs beside the far field: it leaves SMs idle and so does the far field's chain of levels.  Above, both
     // fill the device and sharing it costs more than it hides (measured beside each other: 30,011
     // points, 16 M pairs, 199 against 181 us; a cube of 1e5 points in f64, 58 M, 310 against 289).
     static constexpr int64_t kApartPairs = 200000000;

@@ -1095,12 +1095,12 @@ struct Evaluator final : EvaluatorBase {
             CUDA_TRY(cudaMemsetAsync(Lc.ptr, 0, sizeof(T) * (size_t)m * ms_of(P) * top, stream));
         });
         // On near_stream beside the upward pass: every level's P2L (into Lx), then the
-        // near-singular sums, then (with overlap, or a small plan) the near field, summed apart
+        // near-singular sums, then (set so, or a small plan) the near field, summed apart
         // (it needs only the charges) and added by output_kernel: far + near, the addition of the fused P2P
         // epilogue, so the same floats.
         const bool side = !timer.on;
         const bool x = (kinds & 2) && Lx.ptr;
-        const bool apart = (overlap || near_pairs * m <= kApartPairs) && side && kinds == 3 && items.count;
+        const bool apart = (overlap > 0 || (overlap < 0 && near_pairs * m <= kApartPairs)) && side && kinds == 3 && items.count;
         const bool fork = side && (x || sums || apart);
         if (fork) {
             CUDA_TRY(cudaEventRecord(ev_fork, stream));

@@ -234,10 +234,11 @@ int fmmgpu_fmm_set_graph(fmmgpu_fmm* fmm, int on);
 
 /* Near field beside the far field (on = 1): an evaluation runs P2P on a second,
  * lower-priority stream, concurrently with the far-field passes, and one output pass adds
- * the two (the same addition as the serial order, so the same floats).  0, the default,
- * runs everything on one stream (on one B200 the two halves compete for the same FP32
- * pipes and the overlap measured no faster).  Per-kind timing always runs on one stream.
- * Synchronises. */
+ * the two (the same addition as the serial order, so the same floats).  0 runs the near field
+ * after the far field.  Until the first call the plan's size decides: beside the far field up
+ * to 2e8 near pairs x vectors, where both leave SMs idle; after it above (the two halves then
+ * compete for the same pipes and the overlap measured no faster).  Per-kind timing always runs
+ * on one stream.  Synchronises. */
 int fmmgpu_fmm_set_overlap(fmmgpu_fmm* fmm, int on);
 
 /* Times the launch shapes that change no result on this handle's plan and device and
