@@ -1414,8 +1414,12 @@ struct Evaluator final : EvaluatorBase {
         if (p2p_path == 1) {
             const P2pStream st{st_rowpair.as<int64_t>(), st_xy.as<float4>(), st_zz.as<float2>(), st_idx.as<int2>()};
             if (!gradients) {
-                p2p_st_mv_kernel<W><<<counted(g), 32 * W, 0, s>>>(dp, it, m, near, kRmax, st, q, tp, close,
-                                                                 far_phi.as<double>(), accumulate, d_phi);
+                if (m > kX2Vb)
+                    p2p_st_mv_kernel<W, 2 * kX2Vb><<<counted(g), 32 * W, 0, s>>>(
+                        dp, it, m, near, kRmax, st, q, tp, close, far_phi.as<double>(), accumulate, d_phi);
+                else
+                    p2p_st_mv_kernel<W, kX2Vb><<<counted(g), 32 * W, 0, s>>>(
+                        dp, it, m, near, kRmax, st, q, tp, close, far_phi.as<double>(), accumulate, d_phi);
                 return;
             }
             const P2pStArgs a{dp, it, m, near, kRmax, st, q, tp, close, far_phi.as<double>(), fg, accumulate, d_phi, og};

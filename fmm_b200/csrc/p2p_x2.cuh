@@ -864,17 +864,18 @@ __global__ void __launch_bounds__(32 * W, 32 / W) p2p_st_kernel(P2pStArgs a) {
 void launch_p2p_st(const P2pStArgs& a, int warps, int ks, unsigned grid, cudaStream_t s);
 
 // Potentials of several vectors from the stream: p2p_x2_mv_kernel's pair-steps (the pair
-// geometry once, q rinv added per vector) on flushes copied from the stream.
-template <int W>
+// geometry once, q rinv added per vector) on flushes copied from the stream, for VB vectors at a
+// time: kX2Vb, or twice that for passes of more vectors (a pair's geometry is about 13 of the
+// 13 + 2 VB instructions of a pair-step).  A vector's floats are the same for either.
+template <int W, int VB>
 __global__ void __launch_bounds__(32 * W, 20 / W) p2p_st_mv_kernel(
     DevPlan plan, P2pItems items, int m, int near, float rmax, P2pStream st, const float* __restrict__ sq,
     const float4* __restrict__ tpos, ClosePairs close, double* __restrict__ far_phi, int accumulate,
     double* __restrict__ out_phi) {
-    constexpr int VB = kX2Vb;
     __shared__ float4 sxy[W][2][kStPairs];
     __shared__ float2 szz[W][2][kStPairs];
     __shared__ float2 sqq[W][2][VB][kStPairs];
-    static_assert(VB * 32 * sizeof(double) <= sizeof(float4) * kStPairs, "reduction buffer");
+    static_assert(VB * 32 * sizeof(double) <= VB * sizeof(float2) * kStPairs, "reduction buffer");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t item = (int64_t)blockIdx.x * W + warp;
     if (item >= items.count) return;
@@ -990,7 +991,7 @@ __global__ void __launch_bounds__(32 * W, 20 / W) p2p_st_mv_kernel(
         }
         if (!last) continue;
         if (K > 1) {
-            double(*red)[32] = reinterpret_cast<double(*)[32]>(&sxy[warp][b][0]);
+            double(*red)[32] = reinterpret_cast<double(*)[32]>(&sqq[warp][b][0][0]);  // this flush is read
 #pragma unroll
             for (int vb = 0; vb < VB; ++vb) red[vb][lane] = aphi[vb];
             __syncwarp();
