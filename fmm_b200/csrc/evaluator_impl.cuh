@@ -71,7 +71,7 @@ struct Evaluator final : EvaluatorBase {
     std::vector<int64_t> m2m_tiles, l2l_tiles;  // tile ranges per level (nlevels + 1)
     // the same pairs per level and octant (9 offsets a level) for the chains of small levels
     // (tree_chain.cuh), the M2M parents' ranges on the device, and the pairs of each level
-    DevBuf up_off, down_off, m2m_start_d;
+    DevBuf up_off, down_off, m2m_start_d, m2m_rec;
     std::vector<int64_t> up_pairs, down_pairs;
     // M2L batches: pairs of all levels grouped by offset, in tiles
     DevBuf tile_d, tile_begin, tile_count, pair_e, pair_src, v_pos;
@@ -387,8 +387,8 @@ struct Evaluator final : EvaluatorBase {
                 if constexpr (ChainShape<P, T, CPLX>::OK)
                     timed<CPLX>(kM2M, [&] {
                         chain_up_kernel<P, T, CPLX><<<counted(8), kChainThreads, ChainShape<P, T, CPLX>::SMEM, stream>>>(
-                            dp, ChainPairs{up_off.as<int64_t>(), oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>()},
-                            m2m_par.as<int32_t>(), m2m_start_d.as<int64_t>(), l, l0 + 1, m, tab, tab_level, yo, mm);
+                            ChainPairs{up_off.as<int64_t>(), oct_pair_e.as<int64_t>(), oct_pair_src.as<int32_t>()},
+                            m2m_rec.as<int4>(), m2m_start_d.as<int64_t>(), l, l0 + 1, m, tab, tab_level, yo, mm);
                     });
                 l = l0;
             } else {
@@ -844,6 +844,14 @@ struct Evaluator final : EvaluatorBase {
             (pass == 0 ? up_off : down_off).upload(off);
         }
         m2m_start_d.upload(m2m_start);
+        std::vector<int4> rec(a.size());
+        for (size_t i = 0; i < a.size(); ++i) {
+            const int32_t c0 = plan.child_first[a[i]];
+            int bits = 0;
+            for (int c = 0; c < 8; ++c) bits |= (plan.src_below[c0 + c] > 0) << c;
+            rec[i] = make_int4(a[i], c0, bits, 0);
+        }
+        m2m_rec.upload(rec);
         oct_tile_d.upload(td);
         oct_tile_begin.upload(tb);
         oct_tile_count.upload(tc);
@@ -1071,7 +1079,7 @@ struct Evaluator final : EvaluatorBase {
                                &fu_tile_np, &fu_cta, &fu_pair_src, &fu_pair_tgt, &fu_img, &ck_tc_d, &ck_tc_begin,
                                &ck_tc_count, &ck_s_d, &ck_s_begin, &ck_s_count, &ck_pair_src, &st_rowpair,
                                &st_xy, &st_zz, &st_idx, &close_w, &close_acc, &close_src32, &up_off, &down_off,
-                               &m2m_start_d, &tc_cta, &tc2_cta};
+                               &m2m_start_d, &m2m_rec, &tc_cta, &tc2_cta};
         size_t s = 0;
         for (auto* b : all) s += b->bytes;
         return s;

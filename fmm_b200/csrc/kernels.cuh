@@ -459,12 +459,6 @@ template <typename T>
 __device__ __forceinline__ bool x_of(const DevPlan& plan, int64_t box, const T* Lx) {
     return Lx && plan.x_row[box + 1] > plan.x_row[box];
 }
-template <typename T>
-__device__ __forceinline__ void add_local(T* L, const T* Lx, bool x, T v) {
-    T s = v + __ldcg(L);
-    if (x) s += *Lx;
-    *L = s;
-}
 __device__ __forceinline__ void add_local(double* L, const double* Lx, bool x, double2 v) {
     const double2 u = __ldcg(reinterpret_cast<const double2*>(L));
     v.x += u.x;
@@ -638,9 +632,9 @@ struct GemmShape {
 // Rows: a box holds MV = m (real) or 2m (CPLX: rows 2v and 2v + 1 the real and imaginary
 // planes of vector v) expansion rows of ms_of(P) slots; a product holds MV rows of
 // ys_of(P) slots.
-// ADD: the L2L of a level, Y = the locals: the product is added to the child's row as
-// add_local does (its X sum from Lx).  The vectors are dealt over blockIdx.y (a block a tile
-// with 16 vectors in turn took 80 us for levels of 24 to 104 tiles).
+// ADD: the L2L of a level, Y = the locals: the product is added to the child's row,
+// (T L_parent + S) + X.  The vectors are dealt over blockIdx.y (a block a tile with 16 vectors
+// in turn took 80 us for levels of 24 to 104 tiles).
 template <int P, typename T, bool CPLX = false, bool ADD = false>
 __global__ void __launch_bounds__(256) m2l_gemm_kernel(const int32_t* __restrict__ tile_d,
                                                        const int64_t* __restrict__ tile_begin,
@@ -743,18 +737,26 @@ __global__ void __launch_bounds__(256) m2l_gemm_kernel(const int32_t* __restrict
             if (pr >= cnt) continue;
             const int64_t e = pair_e ? pair_e[p0 + pr] : p0 + pr;
             const bool x = ADD && x_of(plan, e, Lx);
+            auto place = [&](int n) {
+                const int plane = CPLX ? n / NC : 0, slot_ = CPLX ? n % NC : n;
+                return (e * mv + vrow + plane) * ys_of(P) + slot_;
+            };
+            if (ADD)  // a row's locals (and X sums) read together, then added
 #pragma unroll
-            for (int j = 0; j < JN; ++j) {
-                const int n = tx + 16 * j;
-                if (n < NE) {
-                    const int plane = CPLX ? n / NC : 0, slot_ = CPLX ? n % NC : n;
-                    const int64_t at = (e * mv + vrow + plane) * ys_of(P) + slot_;
+                for (int j = 0; j < JN; ++j)
+                    if (tx + 16 * j < NE) acc[i][j] += __ldcg(Y + place(tx + 16 * j));
+            if (x)
+#pragma unroll
+                for (int j = 0; j < JN; ++j)
+                    if (tx + 16 * j < NE) acc[i][j] += Lx[place(tx + 16 * j)];
+#pragma unroll
+            for (int j = 0; j < JN; ++j)
+                if (tx + 16 * j < NE) {
                     if (ADD)
-                        add_local(Y + at, Lx + at, x, acc[i][j]);
+                        Y[place(tx + 16 * j)] = acc[i][j];
                     else  // read once by the reduce: stream past L2
-                        __stcs(Y + at, acc[i][j]);
+                        __stcs(Y + place(tx + 16 * j), acc[i][j]);
                 }
-            }
         }
     }
 }
