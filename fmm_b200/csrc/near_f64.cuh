@@ -55,6 +55,49 @@ __device__ __forceinline__ void inv_dist(const double (&r2)[U], double (&y)[U]) 
             if (__double2hiint(r2[u]) < 0x01000000) y[u] = r2[u] == 0.0 ? 0.0 : rsqrt(r2[u]);
 }
 
+// sin and cos of U phases.  Reduced to [-pi/4, pi/4] by Cody and Waite's two-step subtraction of
+// n pi/2 (pi/2 as a double and the remainder, each step one fma), then the Taylor polynomials to
+// x^17 and x^16, whose remainders there are below 2^-58; at most 1.1e-16 off over [0, 1e5].
+// Branch-free up to |x| = 1e5, so that the pairs' chains overlap; beyond it (and for infinities
+// and NaN) the library's form.  Helmholtz on 40,009 points: 707 -> 682 us against sincos().
+template <int U>
+__device__ __forceinline__ void sin_cos(const double (&x)[U], double (&sn)[U], double (&cs)[U]) {
+    bool far = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const double n = rint(x[u] * 0.63661977236758134);  // 2 / pi
+        double r = __fma_rn(-n, 1.5707963267948966, x[u]);
+        r = __fma_rn(-n, 6.123233995736766e-17, r);  // pi / 2 minus its double
+        const double z = r * r;
+        double s = 1.0 / 355687428096000.0, c = 1.0 / 20922789888000.0;  // 1 / 17!, 1 / 16!
+        s = __fma_rn(s, z, -1.0 / 1307674368000.0);
+        c = __fma_rn(c, z, -1.0 / 87178291200.0);
+        s = __fma_rn(s, z, 1.0 / 6227020800.0);
+        c = __fma_rn(c, z, 1.0 / 479001600.0);
+        s = __fma_rn(s, z, -1.0 / 39916800.0);
+        c = __fma_rn(c, z, -1.0 / 3628800.0);
+        s = __fma_rn(s, z, 1.0 / 362880.0);
+        c = __fma_rn(c, z, 1.0 / 40320.0);
+        s = __fma_rn(s, z, -1.0 / 5040.0);
+        c = __fma_rn(c, z, -1.0 / 720.0);
+        s = __fma_rn(s, z, 1.0 / 120.0);
+        c = __fma_rn(c, z, 1.0 / 24.0);
+        s = __fma_rn(s, z, -1.0 / 6.0);
+        c = __fma_rn(c, z, -0.5);
+        s = __fma_rn(s * z, r, r);
+        c = __fma_rn(c, z, 1.0);
+        const int q = __double2int_rn(n);
+        const double a = q & 1 ? c : s, b = q & 1 ? s : c;
+        sn[u] = q & 2 ? -a : a;
+        cs[u] = (q + 1) & 2 ? -b : b;
+        far |= !(fabs(x[u]) <= 1e5);
+    }
+    if (far)
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (!(fabs(x[u]) <= 1e5)) sincos(x[u], &sn[u], &cs[u]);
+}
+
 // The Laplace pair of VB charge vectors (the geometry formed once).
 template <bool GRAD_, int VB_>
 struct NearLaplace {
@@ -107,21 +150,25 @@ struct NearHelmholtz {
 #pragma unroll
         for (int u = 0; u < U; ++u) r2[u] = pair_r2<double>(d[u][0], d[u][1], d[u][2]);
         inv_dist<U>(r2, y);
+        double r[U], ph[U], sn[U], cs[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            double r = r2[u] * y[u];
-            r = __fma_rn(0.5 * y[u], __fma_rn(-r, r, r2[u]), r);
-            const double phase = k.kre * r;
-            double sn, cs;
-            sincos(phase, &sn, &cs);
-            double damping = 0.0;
-            if (k.kim != 0.0) {
-                damping = -(k.kim * r);
-                const double decay = exp(damping);
-                sn *= decay;
-                cs *= decay;
+            r[u] = r2[u] * y[u];
+            r[u] = __fma_rn(0.5 * y[u], __fma_rn(-r[u], r[u], r2[u]), r[u]);
+            ph[u] = k.kre * r[u];
+        }
+        sin_cos<U>(ph, sn, cs);
+        if (k.kim != 0.0)
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const double decay = exp(-(k.kim * r[u]));
+                sn[u] *= decay;
+                cs[u] *= decay;
             }
-            const double qr = q[u][0] * cs - q[u][1] * sn, qi = q[u][0] * sn + q[u][1] * cs;  // q e
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const double phase = ph[u], damping = -(k.kim * r[u]);
+            const double qr = q[u][0] * cs[u] - q[u][1] * sn[u], qi = q[u][0] * sn[u] + q[u][1] * cs[u];  // q e
             a[0] = __fma_rn(qr, y[u], a[0]);
             a[1] = __fma_rn(qi, y[u], a[1]);
             if (GRAD) {
@@ -167,7 +214,7 @@ constexpr int near_stage_doubles() {  // x, y, z, charges, in 16-byte pairs
 // two pairs in flight instead of four 1.58 to 1.61).
 template <class PK>
 constexpr int near_blocks(bool share) {
-    return share || PK::HELM || PK::VB > 1 ? 1 : 5;
+    return share || PK::VB > 1 ? 1 : PK::HELM ? 3 : 5;
 }
 
 // SHARE: the block's warps share one item (its flushes dealt round robin); else a warp an item.

@@ -59,3 +59,19 @@ def test_long_near_rows_match_oracle(oracle):
     phi, g = oracle.fmm(x, q, x, 5, 4, gradients=True, threads=8)
     assert rel(out.potential, phi) < 1e-12 and rel(out.gradient, g) < 1e-12
     fmm.close()
+
+
+# phases below a quarter turn, over many turns, beyond 1e5 (the library's reduction) and damped.
+# 1e-13 as above plus the phase's own rounding: k r with k, r each rounded, so up to a few
+# 2^-53 k r of a turn's angle (r below 2 in these boxes)
+@pytest.mark.parametrize("k", [0.5, 40.0, 700.0, 4e5, 3.0 + 2.0j])
+def test_helmholtz_phases(k):
+    rng = np.random.default_rng(5)
+    x, t = rng.random((130, 3)), rng.random((57, 3))
+    z = rng.standard_normal((130, 1)) + 1j * rng.standard_normal((130, 1))
+    fmm = F.FmmBuilder(3).gradients().max_points_per_leaf(200).build(x, t)
+    out = fmm.helmholtz_near(k, z)
+    phi, g = direct(x, t, z, k)
+    tol = 1e-13 + 8 * 2.0 ** -53 * abs(k) * 2
+    assert rel(out.potential, phi) < tol and rel(out.gradient, g) < tol
+    fmm.close()
