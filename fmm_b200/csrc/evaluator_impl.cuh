@@ -149,6 +149,7 @@ struct Evaluator final : EvaluatorBase {
     // split its pair-steps, so lanes idle only in the last item); each list in leaf order,
     // with explicit targets and slots, on a kernel with K fixed at compile time.
     static constexpr int kP2pClasses = 4;
+    static constexpr int64_t kOneWarpItems = 32768;
     DevBuf pitem_leaf, pitem_t0, pitem_n;
     P2pItems plist[kP2pClasses]{};
     std::vector<int64_t> plist_lstart[kP2pClasses];  // first item of each level (nlevels + 1)
@@ -919,6 +920,10 @@ struct Evaluator final : EvaluatorBase {
         items.t0 = item_t0.as<int64_t>();
         items.count = (int64_t)il.size();
         build_p2p_lists();
+        // one item a block where the lists fill the device many times over (a finished item frees
+        // its warp's slot at once: 4e6 points of a sphere 1.91 against 2.02 ms, 1e6 of a cube 0.513
+        // against 0.537, a batch of 700,000 with 16 vectors 1.30 against 1.33); four below, where it is even
+        if (kMixed && items.count >= kOneWarpItems) p2p_warps = 1;
     }
 
     // The lists of a leaf's targets by item slots.  f64: one list in leaf order (its kernel

@@ -1005,8 +1005,8 @@ __global__ void __launch_bounds__(128) leaf_far_mv_items_kernel(DevPlan plan, P2
 // target with the vectors in turn, the expansions staged in shared memory behind two block
 // barriers each, kept 5).  Coefficients are read straight from global memory, the same value
 // for every lane of one vector.  Each evaluation's sums do not depend on the other lanes.
-// Bound by the coefficients' loads and the FP64 pipe.  Measured: 41,017 targets x 4 vectors at
-// p = 10 (5 targets a leaf) 0.89 -> 0.27 ms, 1e6 targets at p = 8 0.25 -> 0.10.
+// Bound by the coefficients' loads and the FP64 pipe.  Measured: 1e6 targets at p = 8 0.25 -> 0.10
+// ms; 41,017 targets x 4 vectors at p = 10: see for_rows.
 template <int P, bool GRAD>
 __global__ void __launch_bounds__(128) leaf_far_f64_kernel(DevPlan plan, P2pItems items, int mode, int m,
                                                           const double4* __restrict__ tpos,
