@@ -292,14 +292,14 @@ __global__ void __launch_bounds__(SHARE ? 256 : 32 * kNearWarps, near_blocks<PK>
                 __syncwarp();
             const int tot = rec_pre[rw][kNearRecs];
             const int nfl = (tot + kNearFlush - 1) / kNearFlush;
-            // a lane's two sources of flush f, mapped; past the end: no charge, away from any target
+            // a lane's two sources of flush f, mapped; past the end: the last source without its charge
+            // (a point of the run, so that a growing wave, Im k < 0, is finite there too)
             auto fetch = [&](int f, double (&s)[2][SD]) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const int pos = f * kNearFlush + lane + 32 * h;
+                    const int at = f * kNearFlush + lane + 32 * h, pos = at < tot ? at : tot - 1;
 #pragma unroll
-                    for (int c = 0; c < SD; ++c) s[h][c] = c < 3 ? 1024.0 : 0.0;
-                    if (pos >= tot) continue;
+                    for (int c = 3; c < SD; ++c) s[h][c] = 0.0;
                     int lo = 0;  // the last entry starting at or before pos
 #pragma unroll
                     for (int b = kNearRecs / 2; b; b >>= 1)
@@ -310,6 +310,7 @@ __global__ void __launch_bounds__(SHARE ? 256 : 32 * kNearWarps, near_blocks<PK>
                     s[h][0] = map_coord<double>(fr.w, u.x, fr.x);
                     s[h][1] = map_coord<double>(fr.w, u.y, fr.y);
                     s[h][2] = map_coord<double>(fr.w, u.z, fr.z);
+                    if (at >= tot) continue;
                     if constexpr (HELM) {
                         const double2 q = reinterpret_cast<const double2*>(A.sq)[(int64_t)v0 * plan.nsrc + si];
                         s[h][3] = q.x;

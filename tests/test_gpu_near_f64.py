@@ -75,3 +75,21 @@ def test_helmholtz_phases(k):
     tol = 1e-13 + 8 * 2.0 ** -53 * abs(k) * 2
     assert rel(out.potential, phi) < tol and rel(out.gradient, g) < tol
     fmm.close()
+
+
+# a growing wave (Im k < 0) at source counts on and off the flush size.  In the leaf's half-widths
+# Im k is down to -20: every pair is finite (at most e^(20 sqrt 3)), a point 1,000 half-widths
+# away would not be.  1e-13 as above plus the rounding of the exponent and the phase (|k| r, r below 2)
+@pytest.mark.parametrize("k", [3.0 - 1.0j, -2.0j, 5.0 - 40.0j])
+@pytest.mark.parametrize("ns", [1, 2, 63, 64, 65, 130])
+def test_growing_wave(k, ns):
+    rng = np.random.default_rng(ns)
+    x, t = rng.random((ns, 3)), rng.random((41, 3))
+    z = rng.standard_normal((ns, 1)) + 1j * rng.standard_normal((ns, 1))
+    fmm = F.FmmBuilder(3).gradients().max_points_per_leaf(200).build(x, t)
+    assert fmm.info()["nleaves"] == 1
+    out = fmm.helmholtz_near(k, z)
+    phi, g = direct(x, t, z, k)
+    tol = 1e-13 + 8 * 2.0 ** -53 * abs(k) * 2
+    assert rel(out.potential, phi) < tol and rel(out.gradient, g) < tol
+    fmm.close()
