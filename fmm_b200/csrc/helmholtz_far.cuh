@@ -386,6 +386,8 @@ __global__ void __launch_bounds__(32) hh_expand_kernel(DevPlan plan, HhLevels lv
             __syncwarp();
         }
     }
+    if (first)  // X leaves without a source (a caller's plan may hold them): the row adds nothing
+        for (int i = lane; i < 2 * nv * NC; i += 32) outb[(int64_t)(2 * v0 + i / NC) * MS + i % NC] = T(0);
     }
 }
 
