@@ -48,6 +48,13 @@ __host__ __device__ __forceinline__ uint32_t tf32_round_bits(uint32_t bits) {
     return (bits + 0x1000u) & ~0x1FFFu;
 }
 
+// the low part of a split: the rest x - hi rounded.  A rest that is NaN (x NaN or infinite, and
+// then the NaN the device makes, 0x7FFFFFFF, whose rounding would carry over the sign bit to
+// -0) stays NaN: as a signed number no other value lies above the bound.
+__device__ __forceinline__ uint32_t tf32_low_bits(float rest) {
+    return tf32_round_bits((uint32_t)min(__float_as_int(rest), 0x7FFFEFFF));
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -445,10 +452,10 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
                     hi.y = tf32_round_bits(__float_as_uint(x.y));
                     hi.z = tf32_round_bits(__float_as_uint(x.z));
                     hi.w = tf32_round_bits(__float_as_uint(x.w));
-                    lo.x = tf32_round_bits(__float_as_uint(x.x - __uint_as_float(hi.x)));
-                    lo.y = tf32_round_bits(__float_as_uint(x.y - __uint_as_float(hi.y)));
-                    lo.z = tf32_round_bits(__float_as_uint(x.z - __uint_as_float(hi.z)));
-                    lo.w = tf32_round_bits(__float_as_uint(x.w - __uint_as_float(hi.w)));
+                    lo.x = tf32_low_bits(x.x - __uint_as_float(hi.x));
+                    lo.y = tf32_low_bits(x.y - __uint_as_float(hi.y));
+                    lo.z = tf32_low_bits(x.z - __uint_as_float(hi.z));
+                    lo.w = tf32_low_bits(x.w - __uint_as_float(hi.w));
                     const uint32_t off = cv_off[j] + (uint32_t)(g0 / CV::N) * CV::ROWS * 128u;
                     *reinterpret_cast<uint4*>(xh + off) = hi;
                     *reinterpret_cast<uint4*>(xl + off) = lo;

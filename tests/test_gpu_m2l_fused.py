@@ -94,3 +94,33 @@ def test_pass_holds_at_most_a_tile_of_vectors(oracle):
     with pytest.raises(F.FmmError, match="at most 64"):
         fmm.set_m2l_path(2)
     fmm.close()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("p,m", [(3, 1), (6, 16), (8, 1), (11, 1), (12, 2)])
+def test_a_charge_that_is_no_number_reaches_every_target(oracle, bad, p, m):
+    """One NaN or infinite charge: no target of its vector keeps a finite potential or gradient, on
+    the product path and (to p = 8) the fused one; the other vectors keep their floats."""
+    x, q = oracle.point_sets("cube", 20000, 15)
+    q = _charges(q, m).reshape(len(x), m)
+    fmm = F.FmmBuilder(p).gradients().vectors(m).max_points_per_leaf(32).precision("mixed").build(x)
+    want = fmm.evaluate(q)
+    q[1234, m - 1] = bad
+    for path in (1, 2) if p <= 8 else (1,):
+        fmm.set_m2l_path(path)
+        out = fmm.evaluate(q)
+        assert not np.isfinite(out.potential[m - 1]).any() and not np.isfinite(out.gradient[m - 1]).any()
+        assert np.array_equal(out.potential[:m - 1], want.potential[:m - 1])
+    fmm.close()
+
+
+@pytest.mark.parametrize("p", [3, 8, 10])
+def test_a_helmholtz_charge_that_is_no_number_reaches_every_target(oracle, p):
+    x, q = oracle.point_sets("cube", 8000, 16)
+    z = (q + 0.5j * q[::-1]).astype(np.complex128)
+    z[77] = np.nan
+    fmm = F.FmmBuilder(p).gradients().max_points_per_leaf(32).precision("mixed").build(x)
+    assert fmm.info()["nlevels"] > 3
+    out = fmm.helmholtz_evaluate(4.0, z)
+    assert not np.isfinite(out.potential).any() and not np.isfinite(out.gradient).any()
+    fmm.close()
