@@ -38,8 +38,9 @@ namespace fmmb {
 // its slow-path tests.  Below 2^-1007 (and at 0) the library's form, behind one branch for the
 // U pairs: a branch a pair kept the pairs' dependent chains from overlapping (the FP64 pipe was
 // 39 % busy, the warps waiting on their own results).
+// Returns whether any of them went that way (the only one in which r2 == 0 occurs).
 template <int U>
-__device__ __forceinline__ void inv_dist(const double (&r2)[U], double (&y)[U]) {
+__device__ __forceinline__ bool inv_dist(const double (&r2)[U], double (&y)[U]) {
     bool small = false;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -53,6 +54,7 @@ __device__ __forceinline__ void inv_dist(const double (&r2)[U], double (&y)[U]) 
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (__double2hiint(r2[u]) < 0x01000000) y[u] = r2[u] == 0.0 ? 0.0 : rsqrt(r2[u]);
+    return small;
 }
 
 // sin and cos of U phases.  Reduced to [-pi/4, pi/4] by Cody and Waite's two-step subtraction of
@@ -144,12 +146,19 @@ struct NearHelmholtz {
     struct Const {
         double kre, kim;
     };
-    __device__ static __forceinline__ void pairs(const Const& k, const double (&d)[U][3], const double (&q)[U][Q],
+    __device__ static __forceinline__ void pairs(const Const& k, const double (&d)[U][3], const double (&qs)[U][Q],
                                                  double (&a)[C]) {
-        double r2[U], y[U];
+        double r2[U], y[U], q[U][Q];
 #pragma unroll
-        for (int u = 0; u < U; ++u) r2[u] = pair_r2<double>(d[u][0], d[u][1], d[u][2]);
-        inv_dist<U>(r2, y);
+        for (int u = 0; u < U; ++u) {
+            r2[u] = pair_r2<double>(d[u][0], d[u][1], d[u][2]);
+            q[u][0] = qs[u][0];
+            q[u][1] = qs[u][1];
+        }
+        if (inv_dist<U>(r2, y))
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (r2[u] == 0.0) q[u][0] = q[u][1] = 0.0;  // left out whatever its charge, infinite ones too
         double r[U], ph[U], sn[U], cs[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {

@@ -93,3 +93,20 @@ def test_growing_wave(k, ns):
     tol = 1e-13 + 8 * 2.0 ** -53 * abs(k) * 2
     assert rel(out.potential, phi) < tol and rel(out.gradient, g) < tol
     fmm.close()
+
+
+# a source that coincides with a target is left out of its sums whatever the source's charge
+@pytest.mark.parametrize("bad", [np.nan, np.inf, complex(1.0, -np.inf)])
+@pytest.mark.parametrize("k", [2.0, 2.0 - 0.5j])
+def test_a_coincident_charge_that_is_no_number_is_left_out(bad, k):
+    rng = np.random.default_rng(9)
+    x = rng.random((70, 3))
+    z = rng.standard_normal((70, 1)) + 1j * rng.standard_normal((70, 1))
+    z[13] = bad
+    fmm = F.FmmBuilder(3).gradients().max_points_per_leaf(200).build(x)
+    out = fmm.helmholtz_near(k, z)
+    rest = np.arange(70) != 13
+    phi, g = direct(x[rest], x[13:14], z[rest], k)
+    assert rel(out.potential[:, 13:14], phi) < 1e-13 and rel(out.gradient[:, 13:14], g) < 1e-13
+    assert not np.isfinite(out.potential[:, rest]).any()
+    fmm.close()
