@@ -110,3 +110,30 @@ def test_a_coincident_charge_that_is_no_number_is_left_out(bad, k):
     assert rel(out.potential[:, 13:14], phi) < 1e-13 and rel(out.gradient[:, 13:14], g) < 1e-13
     assert not np.isfinite(out.potential[:, rest]).any()
     fmm.close()
+
+
+def one_pair(t):
+    """Points on a grid of 2^-20 and one source at (2^-20, 2^-20, 2^-20), in one leaf of half-width
+    1/2 at (1/2, 1/2, 1/2): the leaf's coordinates, the pairs' differences and r^2 are exact."""
+    x = np.full((1, 3), 2.0 ** -20)
+    b = F.FmmBuilder(3).gradients().max_points_per_leaf(1 << 20)
+    plan = b.plan(x, t).plan_arrays()
+    plan["lower"], plan["side"] = np.zeros(3), 1.0
+    d = 2.0 * (t - x)
+    return b.upload(plan, x, t), d, (d * d).sum(-1)
+
+
+SCALE = 4.0 * 3.141592653589793 * 0.5  # the kernels' output scale of this leaf, the same double
+
+
+# The term of the gradient, q / r^3 d / (4 pi r_t^2) at k = 0: 1/r^3 is to be as good as a division
+# by r2 r, 8.2e-17 rms; with the product's and the output scale's roundings (4.7e-17 each) 1.05e-16
+def test_helmholtz_gradient_term_keeps_the_precision_of_a_division():
+    rng = np.random.default_rng(3)
+    t = rng.integers(2, 1 << 20, (20000, 3)) / 2.0 ** 20
+    fmm, d, r2 = one_pair(t)
+    out = fmm.helmholtz_near(0.0, np.ones((1, 1)))
+    want = -d / (np.sqrt(r2.astype(np.longdouble)) * r2)[:, None] / np.longdouble(SCALE * 0.5)
+    err = ((out.gradient[0].real - want) / want).astype(float)
+    assert np.sqrt((err * err).mean()) < 1.2e-16
+    fmm.close()
