@@ -126,8 +126,8 @@ def one_pair(t):
 SCALE = 4.0 * 3.141592653589793 * 0.5  # the kernels' output scale of this leaf, the same double
 
 
-# The term of the gradient, q / r^3 d / (4 pi r_t^2) at k = 0: 1/r^3 is to be as good as a division
-# by r2 r, 8.2e-17 rms; with the product's and the output scale's roundings (4.7e-17 each) 1.05e-16
+# The term of the gradient, q / r^3 d / (4 pi r_t^2) at k = 0: 1/r^3 to 6.6e-17 rms (a division by
+# r2 r has 8.2e-17); with the product's and the output scale's roundings (4.7e-17 each) 9.4e-17
 def test_helmholtz_gradient_term_keeps_the_precision_of_a_division():
     rng = np.random.default_rng(3)
     t = rng.integers(2, 1 << 20, (20000, 3)) / 2.0 ** 20
@@ -135,5 +135,5 @@ def test_helmholtz_gradient_term_keeps_the_precision_of_a_division():
     out = fmm.helmholtz_near(0.0, np.ones((1, 1)))
     want = -d / (np.sqrt(r2.astype(np.longdouble)) * r2)[:, None] / np.longdouble(SCALE * 0.5)
     err = ((out.gradient[0].real - want) / want).astype(float)
-    assert np.sqrt((err * err).mean()) < 1.2e-16
+    assert np.sqrt((err * err).mean()) < 1.0e-16
     fmm.close()
