@@ -1288,7 +1288,7 @@ struct Evaluator final : EvaluatorBase {
         expand_kernel<P, T, IRREG, VB><<<counted((unsigned)(r1 - r0)), 32, expand_smem<P, T>(VB), s>>>(
             dp, r0, r1, rows, m, spos.as<T4>(), sq.as<T>(), out);
     }
-    static constexpr int kExpandMost = kMixed ? 16 : 4;
+    static constexpr int kExpandMost = expand_most<P, T>();
     static constexpr bool kBfly = kMixed && P <= 10;
     template <bool IRREG>
     void expand_vectors(int64_t r0, int64_t r1, const int32_t* rows, T* out, cudaStream_t s) {
@@ -1300,12 +1300,16 @@ struct Evaluator final : EvaluatorBase {
                     reinterpret_cast<const float*>(sq.ptr), reinterpret_cast<float*>(out), xrec.as<XRec>());
                 return;
             }
-        if (m == 1)
+        if (m == 1) {
             expand<IRREG, 1>(r0, r1, rows, out, s);
-        else if (m <= 4 || !kMixed)
-            expand<IRREG, 4>(r0, r1, rows, out, s);
-        else
-            expand<IRREG, kExpandMost>(r0, r1, rows, out, s);
+            return;
+        }
+        if constexpr (kExpandMost > 4)
+            if (m <= 4) {
+                expand<IRREG, 4>(r0, r1, rows, out, s);
+                return;
+            }
+        expand<IRREG, kExpandMost>(r0, r1, rows, out, s);
     }
 
     void p2m_rows(int64_t r0, int64_t r1) { expand_vectors<false>(r0, r1, nullptr, M.as<T>(), stream); }

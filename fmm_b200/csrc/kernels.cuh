@@ -103,15 +103,68 @@ __global__ void charge_load_kernel(const double* __restrict__ q_caller, const in
 //
 // The row's sources, taken as one run over its entries, go 32 at a time: each lane forms one
 // source's harmonics (conj X, the slots of harmonics.cuh) into shared memory, then the lanes
-// hold the slots lane, lane + 32, ... and add q S over the 32 sources in order, for VB charge
-// vectors at a time, in registers.  The harmonics are so formed once per source and VB
+// hold the slots lane, lane + 32, ... and add q S over the 32 sources, for VB charge vectors at
+// a time, in registers: four sources in order, the eight fours of a chunk as a tree, the chunks
+// in f64, which rounds no more than a source a lane and a butterfly over the lanes (f32, random
+// signs, in units of 2^-24 of the terms' 2-norm, 32 / 600 sources: 1.04 / 1.11, the butterfly 1.10 /
+// 1.69, one sum over all sources 1.72 / 7.33).  The harmonics are so formed once per source and VB
 // vectors, and a run over the X entries fills the lanes where single leaves of 8 to 24 sources
-// left most of them idle: a batch of 700,000 points with 16 vectors at p = 6 takes 0.09 ms for
-// P2M and 0.44 for P2L, against 0.40 and 1.50 with the harmonics formed again for each vector
-// (in f64, whose shared-memory rows of 32 fell in one bank, P2M of 1e6 points at p = 8 takes
-// 0.08 ms against 0.20).  A vector's sums are the same floats for any VB.
+// left most of them idle: a batch of 700,000 points with 16 vectors at p = 6 takes 0.14 ms for
+// P2M and 0.53 for P2L (one sum over all sources: 0.09 and 0.44), against 0.40 and 1.50 with the
+// harmonics formed again for each vector (in f64, whose shared-memory rows of 32 fell in one
+// bank, P2M of 1e6 points at p = 8 takes 0.09 ms against 0.20).  A vector's sums are the same
+// floats for any VB.
 // A handle of one f32 vector keeps the register form below where it is the faster one.
 // ---------------------------------------------------------------------------------
+// A lane's partial sums of a chunk: slots lane, lane + 32, ... of VB vectors
+template <typename T, int NCL, int VB>
+struct ChunkSum {
+    using T2 = typename Pair2<T>::type;
+    T2 v[NCL][(VB + 1) / 2];
+    __device__ __forceinline__ T at(int c, int b) const { return b & 1 ? v[c][b / 2].y : v[c][b / 2].x; }
+    // this + o, or o (first)
+    __device__ __forceinline__ void add(const ChunkSum& o, bool plus) {
+#pragma unroll
+        for (int c = 0; c < NCL; ++c)
+#pragma unroll
+            for (int b = 0; b < (VB + 1) / 2; ++b) v[c][b] = plus ? add2(v[c][b], o.v[c][b]) : o.v[c][b];
+    }
+    // sources j0 .. j0 + 3 in order from zero
+    template <int NC, int SR>
+    __device__ __forceinline__ void four(const T* S, const T* Q, int lane, int j0) {
+#pragma unroll
+        for (int c = 0; c < NCL; ++c)
+#pragma unroll
+            for (int b = 0; b < (VB + 1) / 2; ++b) v[c][b] = mk2(T(0), T(0));
+#pragma unroll
+        for (int j = j0; j < j0 + 4; ++j) {
+            T s[NCL];
+#pragma unroll
+            for (int c = 0; c < NCL; ++c) s[c] = S[(lane + 32 * c < NC ? lane + 32 * c : 0) * SR + j];
+            if constexpr (VB == 1) {
+                const T q = Q[j];
+#pragma unroll
+                for (int c = 0; c < NCL; ++c) v[c][0].x = fma1(q, s[c], v[c][0].x);
+            } else {
+                const T2* q2 = reinterpret_cast<const T2*>(Q + j * VB);
+#pragma unroll
+                for (int b = 0; b < VB / 2; ++b) {
+                    const T2 q = q2[b];
+#pragma unroll
+                    for (int c = 0; c < NCL; ++c) v[c][b] = fma2(q, x2(s[c]), v[c][b]);
+                }
+            }
+        }
+    }
+};
+
+// the most vectors a pass: as many as keep their partial sums in registers (700,000 points with 16
+// vectors at p = 6, P2M and P2L: 8 vectors 0.14 and 0.53 ms, 4 0.14 and 0.61, two passes of 8 over one
+// chunk's harmonics 0.17 and 0.58)
+template <int P, typename T>
+constexpr int expand_most() {
+    return sizeof(T) == 4 ? (P <= 8 ? 8 : 4) : P <= 7 ? 4 : 2;
+}
 template <int P, typename T>
 constexpr int expand_smem(int vb) {
     return (int)sizeof(T) * ((nc_of(P) * 33 + 3) / 4 * 4 + 32 * vb);
@@ -140,11 +193,11 @@ __global__ void __launch_bounds__(32) expand_kernel(DevPlan plan, int64_t row_be
     if (IRREG ? x0 == x1 : plan.src_start[row + 1] == plan.src_start[row]) return;
     for (int v0 = 0; v0 < m; v0 += VB) {
         const int nb = m - v0 < VB ? m - v0 : VB;
-        T2 acc[NCL][(VB + 1) / 2];
+        double run[NCL][VB];  // the finished chunks
 #pragma unroll
         for (int c = 0; c < NCL; ++c)
 #pragma unroll
-            for (int b = 0; b < (VB + 1) / 2; ++b) acc[c][b] = mk2(T(0), T(0));
+            for (int b = 0; b < VB; ++b) run[c][b] = 0.0;
         for (int64_t e0 = x0; e0 < x1; e0 += 32) {
             const int ne = x1 - e0 < 32 ? (int)(x1 - e0) : 32;
             int64_t first = 0;  // P2M: the leaf's first source
@@ -180,65 +233,64 @@ __global__ void __launch_bounds__(32) expand_kernel(DevPlan plan, int64_t row_be
                 tot = (int)(plan.src_start[row + 1] - first);
             }
             for (int cb = 0; cb < tot; cb += 32) {
-                const int pos = cb + lane;
-                if (pos < tot) {
-                    int64_t si = first + pos;
-                    T4 f;
-                    if constexpr (IRREG) {
-                        int lo = 0;  // the last entry starting at or before pos
+                // past the end: the last source, uncharged
+                const int pos = cb + lane < tot ? cb + lane : tot - 1;
+                int64_t si = first + pos;
+                T4 f;
+                if constexpr (IRREG) {
+                    int lo = 0;  // the last entry starting at or before pos
 #pragma unroll
-                        for (int b = 16; b; b >>= 1)
-                            if (lo + b < ne && ent_pre[lo + b] <= pos) lo += b;
-                        f = ent_frame[lo];
-                        si = ent_s0[lo] + (pos - ent_pre[lo]);
-                    }
-                    const T4 p4 = spos[si];
+                    for (int b = 16; b; b >>= 1)
+                        if (lo + b < ne && ent_pre[lo + b] <= pos) lo += b;
+                    f = ent_frame[lo];
+                    si = ent_s0[lo] + (pos - ent_pre[lo]);
+                }
+                const T4 p4 = spos[si];
 #pragma unroll
-                    for (int b = 0; b < VB; ++b)
-                        Q[lane * VB + b] = b < nb ? sq[(int64_t)(v0 + b) * plan.nsrc + si] : T(0);
-                    auto slots = [&](auto& h) {
+                for (int b = 0; b < VB; ++b)
+                    Q[lane * VB + b] = b < nb && cb + lane < tot ? sq[(int64_t)(v0 + b) * plan.nsrc + si] : T(0);
+                auto slots = [&](auto& h) {
 #pragma unroll
-                        for (int n = 0; n <= P; ++n) {
-                            h.step(n);
+                    for (int n = 0; n <= P; ++n) {
+                        h.step(n);
 #pragma unroll
-                            for (int mm = 0; mm <= n; ++mm) {
-                                S[slot(n, mm) * SR + lane] = h.c[mm].x;
-                                if (mm) S[slot(n, -mm) * SR + lane] = -h.c[mm].y;
-                            }
+                        for (int mm = 0; mm <= n; ++mm) {
+                            S[slot(n, mm) * SR + lane] = h.c[mm].x;
+                            if (mm) S[slot(n, -mm) * SR + lane] = -h.c[mm].y;
                         }
-                    };
-                    if constexpr (IRREG) {
-                        const T x = (p4.x - f.x) * f.w, y = (p4.y - f.y) * f.w, z = (p4.z - f.z) * f.w;
-                        IrregularRows2<P, T> h;
-                        h.init(x, y, z, T(1) / sqrt(x * x + y * y + z * z));
-                        slots(h);
-                    } else {
-                        RegularRows2<P, T> h;
-                        h.init(p4.x, p4.y, p4.z);
-                        slots(h);
                     }
+                };
+                if constexpr (IRREG) {
+                    const T x = (p4.x - f.x) * f.w, y = (p4.y - f.y) * f.w, z = (p4.z - f.z) * f.w;
+                    IrregularRows2<P, T> h;
+                    h.init(x, y, z, T(1) / sqrt(x * x + y * y + z * z));
+                    slots(h);
+                } else {
+                    RegularRows2<P, T> h;
+                    h.init(p4.x, p4.y, p4.z);
+                    slots(h);
                 }
                 __syncwarp();
                 const int cnt = tot - cb < 32 ? tot - cb : 32;
-#pragma unroll 2
-                for (int j = 0; j < cnt; ++j) {
-                    T s[NCL];
+                ChunkSum<T, NCL, VB> all;
+#pragma unroll 1
+                for (int h = 0; h < cnt; h += 16) {
+                    ChunkSum<T, NCL, VB> half;
 #pragma unroll
-                    for (int c = 0; c < NCL; ++c) s[c] = S[(lane + 32 * c < NC ? lane + 32 * c : 0) * SR + j];
-                    if constexpr (VB == 1) {
-                        const T q = Q[j];
-#pragma unroll
-                        for (int c = 0; c < NCL; ++c) acc[c][0].x = fma1(q, s[c], acc[c][0].x);
-                    } else {
-                        const T2* q2 = reinterpret_cast<const T2*>(Q + j * VB);
-#pragma unroll
-                        for (int b = 0; b < VB / 2; ++b) {
-                            const T2 q = q2[b];
-#pragma unroll
-                            for (int c = 0; c < NCL; ++c) acc[c][b] = fma2(q, x2(s[c]), acc[c][b]);
-                        }
+                    for (int e = 0; e < 16; e += 8) {
+                        if (h + e >= cnt) break;
+                        ChunkSum<T, NCL, VB> a, b;
+                        a.template four<NC, SR>(S, Q, lane, h + e);
+                        b.template four<NC, SR>(S, Q, lane, h + e + 4);
+                        a.add(b, true);
+                        half.add(a, e != 0);
                     }
+                    all.add(half, h != 0);
                 }
+#pragma unroll
+                for (int c = 0; c < NCL; ++c)
+#pragma unroll
+                    for (int b = 0; b < VB; ++b) run[c][b] += (double)all.at(c, b);
                 __syncwarp();
             }
         }
@@ -248,7 +300,7 @@ __global__ void __launch_bounds__(32) expand_kernel(DevPlan plan, int64_t row_be
             if (k >= NC) break;
 #pragma unroll
             for (int b = 0; b < VB; ++b)
-                if (b < nb) out[((int64_t)box * m + v0 + b) * ms_of(P) + k] = b & 1 ? acc[c][b / 2].y : acc[c][b / 2].x;
+                if (b < nb) out[((int64_t)box * m + v0 + b) * ms_of(P) + k] = (T)run[c][b];
         }
     }
 }
@@ -261,7 +313,7 @@ __global__ void __launch_bounds__(32) expand_kernel(DevPlan plan, int64_t row_be
 // is fixed (per-lane partial sums, then a fixed tree), so results are repeatable.  It serves
 // handles of one vector: P2M to p = 10 (above, its (p+1)^2 sums exceed the register file: 0.19
 // against 0.08 ms for 1e6 points at p = 11) and P2L to p = 10 (4e6 points of a sphere at p = 8
-// 0.22 against 0.31 ms; at p = 11 0.20 against 0.16).
+// 0.22 against 0.30 ms; at p = 11 0.20 against 0.16).
 // ---------------------------------------------------------------------------------
 // One X-list entry of the f32 P2L, fixed at build (x_record_kernel): the source leaf's
 // frame seen from the target box, (c(t|s), r(t|s)) of rel_frame<float>, and its sources,

@@ -31,3 +31,24 @@ def test_leaf_passes_match_oracle(oracle, precision, tol, p, leaf, m):
     lv = fmm.evaluate_levels(q)
     assert np.array_equal(lv.potential, out.potential) and np.array_equal(lv.gradient, out.gradient)
     fmm.close()
+
+
+# P2L rows of about 17,000 sources of one sign, far field alone, in f32 against f64 at the same order:
+# f32's roundings are 1.7e-7 (p = 6, 2 vectors) to 2.8e-7 (p = 11) when a row's sum adds next to nothing
+# to them, 5.5e-7 to 6.5e-7 when it runs over the sources one after another
+@pytest.mark.parametrize("p,m,tol", [(6, 2, 3e-7), (6, 16, 3e-7), (11, 1, 4e-7)])
+def test_long_rows_keep_their_precision(p, m, tol):
+    rng = np.random.default_rng(1)
+    x, t = rng.random((57000, 3)), rng.random((230000, 3))
+    x[:, 0] *= 0.5  # coarse leaves of about 1,800 sources beside finer ones of targets
+    t[:, 0] = 0.5 + 0.5 * t[:, 0]
+    q = rng.random((len(x), m))
+    out = []
+    for precision in ("f64", "mixed"):
+        fmm = F.FmmBuilder(p).vectors(m).max_points_per_leaf(2100).precision(precision).build(x, t)
+        assert fmm.info()["x_pairs"] > 500
+        fmm.set_kinds(2)
+        out.append(fmm.evaluate(q).potential[:, (t[:, 0] > 0.625) & (t[:, 0] < 0.75)])
+        fmm.close()
+    err = (out[1] - out[0]) / out[0]
+    assert np.sqrt((err * err).mean(axis=1)).max() < tol
