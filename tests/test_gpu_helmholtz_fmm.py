@@ -102,3 +102,28 @@ def test_complex64_call_is_the_complex128_call_rounded(cloud, precision):
     assert np.array_equal(got.potential, want.potential.astype(np.complex64))
     assert np.array_equal(got.gradient, want.gradient.astype(np.complex64))
     fmm.close()
+
+
+@pytest.mark.parametrize("p", [10, 11])
+def test_local_expansions_keep_their_precision(p):
+    """A unit source at a leaf's centre, targets within 0.11 half-widths of the centres of leaves two
+    and three away: one translation and L2P, cut off below 1e-16 of the potential at this k.  The
+    error is rounding: 2.5e-16 rms with a sum per degree in L2P (2.3e-16 with three sums over the
+    degrees), 3.5e-16 with one sum over all coefficients; the bound lies between."""
+    rng = np.random.default_rng(2)
+    c = (np.stack(np.meshgrid(*[np.arange(4)] * 3, indexing="ij"), -1).reshape(-1, 3) + 0.5) / 4
+    t = np.repeat(c, 100, axis=0) + np.round((rng.random((6400, 3)) * 2 - 1) * 0.11 / 8 * 2 ** 20) / 2 ** 20
+    x, k = np.full((1, 3), 0.125), 8.0
+    b = F.FmmBuilder(p).gradients().max_points_per_leaf(150).precision("f64")
+    plan = b.plan(x, t).plan_arrays()
+    plan["lower"], plan["side"] = np.zeros(3), 1.0  # the leaves' centres exactly at the grid's
+    fmm = b.upload(plan, x, t)
+    assert fmm.info()["nleaves"] == 64
+    phi = fmm.helmholtz_evaluate(k, np.ones((1, 1))).potential[0]
+    far = np.floor(t * 4).max(axis=1) >= 2
+    r = np.sqrt(((t - x).astype(np.longdouble) ** 2).sum(axis=1))
+    scale = 4 * np.longdouble("3.14159265358979323846264") * r
+    err = np.hypot(phi.real - np.cos(k * r) / scale, phi.imag - np.sin(k * r) / scale).astype(float)
+    want = (1 / scale).astype(float)
+    assert np.sqrt((err[far] ** 2).sum() / (want[far] ** 2).sum()) < 2.9e-16
+    fmm.close()
