@@ -780,6 +780,7 @@ int fmmgpu_fmm_vjp(fmmgpu_fmm* f, const double* charges, const double* cotangent
                                     true);
                 build_device(t.get(), us, ut);
                 t->symmetric = true;  // never asked for its own transpose
+                t->eval->overlap = f->eval->overlap;
                 f->transpose = t.release();
             }
             T = f->transpose;
@@ -1089,6 +1090,11 @@ int fmmgpu_fmm_set_overlap(fmmgpu_fmm* f, int on) {
         CUDA_TRY(cudaStreamSynchronize(f->stream));
         f->eval->overlap = on != 0 ? 1 : 0;
         f->drop_graph();
+        if (f->transpose) {  // a VJP's second evaluation goes by the same choice
+            CUDA_TRY(cudaStreamSynchronize(f->transpose->stream));
+            f->transpose->eval->overlap = f->eval->overlap;
+            f->transpose->drop_graph();
+        }
     });
 }
 

@@ -118,3 +118,37 @@ def test_stored_forward_pass_gives_the_same_vjp(precision, symmetric):
     assert st.info()["vjp_forward_reused"] == 2
     ref.close()
     st.close()
+
+
+@pytest.mark.parametrize("precision", ["f64", "mixed"])
+def test_overlap_choice_holds_for_both_evaluations(precision):
+    """set_overlap governs the second evaluation of a VJP (sources and targets apart) too, whether it is
+    set before the first call or after: near field and far field apart end in output_kernel, the near
+    field after the far field does not."""
+    torch = pytest.importorskip("torch")
+    from torch.profiler import ProfilerActivity, profile
+
+    rng = np.random.default_rng(12)
+    x, t = rng.random((3000, 3)), rng.random((2000, 3))
+    q, w = rng.standard_normal(3000), rng.standard_normal(2000)
+
+    def outputs(fmm):
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            got = fmm.vjp(q, w)
+            torch.cuda.synchronize()
+        names = [e.name for e in prof.events()]
+        assert any("charge_load" in n for n in names)
+        return sum("output_kernel" in n for n in names), got
+
+    b = F.FmmBuilder(4).gradients().max_points_per_leaf(32).precision(precision)
+    want = None
+    for first in (False, True):
+        fmm = b.build(x, t)
+        for on in (first, not first):
+            fmm.set_overlap(on)
+            n, got = outputs(fmm)
+            assert n == (2 if on else 0)
+            want = want or got
+            assert all(np.array_equal(g, v) for g, v in zip(got, want))
+        fmm.close()
