@@ -39,8 +39,9 @@ struct HhState {
     bool built = false;
     // the mixed form's tensor-core M2L (p <= 10): tiles over every level, (level, offset,
     // half) as the table index, the table images, and the multipoles' tensor maps
-    DevBuf tc_d, tc_begin, tc_count, tc_cta, tc_img;
+    DevBuf tc_d, tc_begin, tc_count, tc_cta, tc_img, tc_src;
     int64_t tc_ntiles = 0;
+    int tc_cols = 0;  // columns of a pair of those tiles, of the pair's 2 m
     CUtensorMap mmap{}, vmap{};
 };
 
@@ -1643,7 +1644,28 @@ struct Evaluator final : EvaluatorBase {
             Tiles all, lvl;
             std::vector<int64_t> pe, lstart;
             std::vector<int32_t> ps;
-            batches(std::max(1, S::NT / (2 * m)), all, lvl, lstart, pe, ps);
+            // A pair's 2 m rows follow each other in the multipoles and in the products.  Where they
+            // are more than a tile's columns, the pair is listed as `parts` pairs of 2 m / parts rows.
+            int parts = 1;
+            while (2 * m % parts || 2 * m / parts > S::NT) ++parts;
+            hh.tc_cols = 2 * m / parts;
+            const int tile = S::NT / hh.tc_cols;
+            batches(tile, all, lvl, lstart, pe, ps);
+            if (parts > 1) {
+                Tiles o;
+                std::vector<int64_t> seg(lstart.size(), 0);
+                for (size_t l = 0; l + 1 < lstart.size(); ++l) {
+                    seg[l] = (int64_t)o.d.size();
+                    for (int64_t i = lstart[l]; i < lstart[l + 1]; ++i)
+                        o.add(lvl.d[i], lvl.begin[i] * parts, (int64_t)lvl.count[i] * parts, tile);
+                }
+                seg.back() = (int64_t)o.d.size();
+                lvl = std::move(o);
+                lstart = std::move(seg);
+            }
+            std::vector<int32_t> rows(ps.size() * parts);
+            for (size_t i = 0; i < rows.size(); ++i) rows[i] = ps[i / parts] * parts + (int32_t)(i % parts);
+            hh.tc_src.upload(rows);
             tc_halves_force(lvl, lstart);
             for (int l = 0; l < plan.nlevels; ++l)
                 for (int64_t i = lstart[l]; i < lstart[l + 1]; ++i) lvl.d[i] += (l - 2) * 316 * 2;
@@ -1652,9 +1674,9 @@ struct Evaluator final : EvaluatorBase {
             hh.tc_d.upload(lvl.d);
             hh.tc_begin.upload(lvl.begin);
             hh.tc_count.upload(lvl.count);
-            const int64_t rows = (int64_t)plan.nboxes() * 2 * m;
-            encode_multipole_map<P>(&hh.mmap, reinterpret_cast<const float*>(hh.M.ptr), rows);
-            encode_multipole_map<P>(&hh.vmap, reinterpret_cast<const float*>(hh.M.ptr), rows, 2 * m);
+            const int64_t nrows = (int64_t)plan.nboxes() * 2 * m;
+            encode_multipole_map<P>(&hh.mmap, reinterpret_cast<const float*>(hh.M.ptr), nrows);
+            encode_multipole_map<P>(&hh.vmap, reinterpret_cast<const float*>(hh.M.ptr), nrows, hh.tc_cols);
             CUDA_TRY(cudaFuncSetAttribute(m2l_tc_kernel<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           S::SMEM));
         }
@@ -1729,7 +1751,7 @@ struct Evaluator final : EvaluatorBase {
                 const unsigned grid = (unsigned)std::min<int64_t>(hh.tc_ntiles, num_sms);
                 m2l_tc_kernel<P, true><<<counted(grid), 32 * kTcWarps, TcTs<P, true>::SMEM, stream>>>(
                     hh.tc_d.as<int32_t>(), hh.tc_begin.as<int64_t>(), hh.tc_count.as<int32_t>(), hh.tc_ntiles,
-                    hh.tc_cta.as<int64_t>(), pair_src.as<int32_t>(), 2 * m, hh.tc_img.as<uint32_t>(), hh.mmap, hh.vmap,
+                    hh.tc_cta.as<int64_t>(), hh.tc_src.as<int32_t>(), hh.tc_cols, hh.tc_img.as<uint32_t>(), hh.mmap, hh.vmap,
                     reinterpret_cast<float*>(hh.Y.ptr), tc_error.as<int>());
             }
         } else {

@@ -44,3 +44,40 @@ def test_helmholtz_chain_and_wide_levels_same_floats(oracle, precision, p):
     tol = 0.0 if precision == "f64" else 5e-6
     assert np.linalg.norm(got.potential - want.potential) <= tol * np.linalg.norm(want.potential)
     two.close()
+
+
+@pytest.mark.parametrize("precision", ["f64", "mixed"])
+def test_helmholtz_leaf_sums_of_many_vectors(oracle, precision):
+    """P2M and P2L stage 64 vectors' charges at a time, and a tile of the mixed M2L holds 128 columns, two
+    a vector: 65 to 130 vectors a pass give the floats of 10 a pass."""
+    x, q = oracle.point_sets("sphere", 2500, 3)
+    m = 130
+    z = np.stack([(q + 1j * q[::-1]) * (v + 1.0) * (-1) ** v for v in range(m)], axis=1)
+    b = F.FmmBuilder(3).gradients().max_points_per_leaf(12).precision(precision).vectors(m)
+    out = []
+    for passes in (10, 65, 130):
+        fmm = b.vectors_per_pass(passes).build(x)
+        assert fmm.info()["x_pairs"] > 0
+        if precision == "f64":
+            assert fmm.info()["vectors_per_pass"] == passes
+        o = fmm.helmholtz_evaluate(3.0, z)
+        out.append((o.potential, o.gradient))
+        fmm.close()
+    for potential, gradient in out[1:]:
+        assert np.array_equal(potential, out[0][0]) and np.array_equal(gradient, out[0][1])
+
+
+@pytest.mark.parametrize("p,m,few", [(8, 49, 7), (8, 67, 1), (10, 33, 3)])
+def test_helmholtz_vectors_beyond_one_tile(oracle, p, m, few):
+    """Twice the vectors are more than a tile's columns (96 at p = 8, 64 at p = 10)."""
+    x, q = oracle.point_sets("sphere", 2500, 4)
+    z = np.stack([(q + 1j * q[::-1]) * (v + 1.0) for v in range(m)], axis=1)
+    b = F.FmmBuilder(p).max_points_per_leaf(40).precision("mixed").vectors(m)
+    one, many = b.vectors_per_pass(few).build(x), b.vectors_per_pass(m).build(x)
+    assert many.info()["vectors_per_pass"] == m
+    want, got = one.helmholtz_evaluate(3.0, z).potential, many.helmholtz_evaluate(3.0, z).potential
+    # a vector a pass has another near-field kernel in the mixed form
+    tol = 5e-6 if few == 1 else 0.0
+    assert np.linalg.norm(got - want) <= tol * np.linalg.norm(want)
+    one.close()
+    many.close()
