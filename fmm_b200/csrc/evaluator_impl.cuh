@@ -1153,7 +1153,7 @@ struct Evaluator final : EvaluatorBase {
     // launch count as a plain evaluation does.
     int64_t product_chunks() const override { return (int64_t)chunks.size(); }
     int m2l_tile_columns(int tile) const override {
-        if constexpr (kTensor) return tile ? kTcAlt : TcTs<P>::NT;
+        if constexpr (kTensor) return tile && m <= kTcAlt ? kTcAlt : TcTs<P>::NT;
         return 0;
     }
 
@@ -1214,6 +1214,7 @@ struct Evaluator final : EvaluatorBase {
             float best = 0.f;
             int pick = m2l_tile;
             for (int t : {0, 1}) {
+                if (t == 1 && m > kTcAlt) break;
                 m2l_tile = t;
                 const float ms = time([&] { m2l_products(-1); });
                 if (t == 0 || ms < best) best = ms, pick = t;
@@ -1352,7 +1353,7 @@ struct Evaluator final : EvaluatorBase {
     void m2l_products(int l) {
         if (kTensor && m2l_path == 1) {
             if constexpr (kTensor) {
-                const bool alt = m2l_tile == 1;
+                const bool alt = m2l_tile == 1 && m <= kTcAlt;  // (a pair's m columns in one tile)
                 const std::vector<int64_t>& ls = alt ? tc2_lvl_tiles : tc_lvl_tiles;
                 const int64_t t0 = l < 0 ? 0 : ls[l];
                 const int64_t nt = l < 0 ? (alt ? tc2_ntiles : tc_ntiles) : ls[l + 1] - ls[l];

@@ -59,3 +59,21 @@ def test_p8_alternative_tile_same_bits(oracle):
     alt = fmm.evaluate(q)
     assert np.array_equal(alt.potential, out.potential) and np.array_equal(alt.gradient, out.gradient)
     fmm.close()
+
+
+@pytest.mark.parametrize("p,m", [(6, 65), (8, 81), (9, 33), (11, 47)])
+def test_more_vectors_than_the_alternative_tile_holds(oracle, p, m):
+    """A pass of more vectors than the alternative tile's columns stays on the default tile, set so or
+    tuned."""
+    x, q = oracle.point_sets("sphere", 3000, 30)
+    qs = np.stack([q * (v + 1.0) for v in range(m)], axis=1)
+    fmm = F.FmmBuilder(p).vectors(m).vectors_per_pass(m).max_points_per_leaf(32).precision("mixed").build(x)
+    columns = fmm.info()["m2l_tile_columns"]
+    assert fmm.info()["vectors_per_pass"] == m <= columns
+    want = fmm.evaluate(qs).potential
+    fmm.set_m2l_tile(1)
+    assert fmm.info()["m2l_tile_columns"] == columns
+    assert np.array_equal(fmm.evaluate(qs).potential, want)
+    fmm.autotune(qs)
+    assert np.array_equal(fmm.evaluate(qs).potential, want)
+    fmm.close()
