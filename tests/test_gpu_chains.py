@@ -10,6 +10,27 @@ import fmm_b200 as F
 pytestmark = pytest.mark.gpu
 
 
+CHAIN_ROWS = 1024  # children x vectors of a level up to which it stays in a chain
+
+
+def both_forms(fmm, few, many):
+    """Whether some level of the tree (boxes over a source, below the root) stays in a chain with
+    `few` vectors a pass and runs wide with `many`."""
+    plan = fmm.plan_arrays()
+    keys = plan["keys"].astype(np.uint64)
+    level = (keys & np.uint64(0x7FFF)).astype(int)
+    leaves = np.flatnonzero(plan["is_leaf"])
+    used = keys[leaves[np.diff(plan["source_offsets"].astype(np.int64)) > 0]]
+    count = np.zeros(level.max() + 1, dtype=int)
+    for l in range(level.max(), 0, -1):  # the used boxes of level l, then their parents
+        at = (used & np.uint64(0x7FFF)) == l
+        here = np.unique(used[at])
+        count[l] = len(here)
+        shift = np.uint64(15 + 3 * (16 - (l - 1)))
+        used = np.concatenate([used[~at], ((here >> shift) << shift) | np.uint64(l - 1)])
+    return any(c * few <= CHAIN_ROWS < c * many for c in count[3:])
+
+
 @pytest.mark.parametrize("precision", ["f64", "mixed"])
 @pytest.mark.parametrize("p,n,leaf", [(3, 9000, 8), (6, 9000, 12), (8, 6000, 16), (12, 2500, 16)])
 def test_chain_and_wide_levels_same_floats(oracle, precision, p, n, leaf):
@@ -24,6 +45,7 @@ def test_chain_and_wide_levels_same_floats(oracle, precision, p, n, leaf):
     assert np.array_equal(got.potential, want.potential)
     lv = many.evaluate_levels(qs)
     assert np.array_equal(lv.potential, want.potential)
+    assert both_forms(many, 1, 8)
     many.close()
 
 
@@ -40,10 +62,26 @@ def test_helmholtz_chain_and_wide_levels_same_floats(oracle, precision, p):
     two = b.vectors_per_pass(5).build(x)
     got = two.helmholtz_evaluate(5.0, zs)
     # the near field of one vector runs on another kernel in the mixed form: 5e-6 there (f32
-    # pairs), the same floats in f64
+    # pairs; the levels' floats are compared below), the same floats in f64
     tol = 0.0 if precision == "f64" else 5e-6
     assert np.linalg.norm(got.potential - want.potential) <= tol * np.linalg.norm(want.potential)
     two.close()
+
+
+@pytest.mark.parametrize("precision,p", [("f64", 4), ("f64", 8), ("mixed", 4), ("mixed", 10), ("mixed", 12)])
+def test_helmholtz_levels_same_floats_whatever_the_pass(oracle, precision, p):
+    x, q = oracle.point_sets("sphere", 5000, p)
+    z = q + 1j * q[::-1]
+    b = F.FmmBuilder(p).gradients().max_points_per_leaf(16).precision(precision).vectors(8)
+    zs = np.stack([z * (v + 1.0) for v in range(8)], axis=1)
+    few = b.vectors_per_pass(2).build(x)  # two, not one: the near field's kernel is then the same
+    assert both_forms(few, 2, 8)
+    want = few.helmholtz_evaluate(5.0, zs)
+    few.close()
+    many = b.vectors_per_pass(8).build(x)
+    got = many.helmholtz_evaluate(5.0, zs)
+    assert np.array_equal(got.potential, want.potential) and np.array_equal(got.gradient, want.gradient)
+    many.close()
 
 
 @pytest.mark.parametrize("precision", ["f64", "mixed"])
