@@ -130,9 +130,12 @@ struct EvaluatorBase {
     // near field on its own stream beside the far field: 1 on, 0 off (set_overlap), -1 by size
     int overlap = -1;
     int64_t near_pairs = 0;  // of the plan
-    // By size, the near field of at most this many pairs and vectors runs beside the far field: it leaves SMs idle and so does the far field's chain of levels.  Above, both
-    // fill the device and sharing it costs more than it hides (measured beside each other: 30,011
-    // points, 16 M pairs, 199 against 181 us; a cube of 1e5 points in f64, 58 M, 310 against 289).
+    // By size, the near field of at most this many pairs x vectors runs beside the far field, whose
+    // chain of levels and launches leaves SMs idle.  Measured beside against after, 118 plans of
+    // cubes, spheres and clusters, p = 4 to 8, 1 and 4 vectors, f64 and mixed (graph replay): below the
+    // limit 0.68 to 1.00 of the time (two plans 1.02 and 1.04), above it 0.84 to 1.00 up to 6e8 pairs
+    // and 0.89 to 1.045 beyond, where the two halves compete for the same pipes.  The gains are the
+    // small plans', and the limit keeps clear of the losses.
     static constexpr int64_t kApartPairs = 200000000;
     // launch shapes the autotuner may change: warps a block of the mixed P2P kernel
     // (1, 2 or 4) and threads a block of the L2P / M2P kernel (32, 64 or 128)

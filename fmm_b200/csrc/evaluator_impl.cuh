@@ -142,7 +142,6 @@ struct Evaluator final : EvaluatorBase {
     cudaStream_t near_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_x = nullptr, ev_join = nullptr;
     P2pItems items{};
-    std::vector<int64_t> item_lstart;  // first work item of each level's leaves (nlevels + 1)
     std::vector<int32_t> item_leaf_h;  // the items' leaves (host copy, ascending)
     // The mixed P2P's own work lists, by item slots: every item of 32 targets (one target a
     // lane), then the remainders of the leaves cut into items of 16 and of 8 targets and a
@@ -909,11 +908,6 @@ struct Evaluator final : EvaluatorBase {
                 il.push_back((int32_t)j);
                 it.push_back(t);
             }
-        item_lstart.assign(plan.nlevels + 1, (int64_t)il.size());
-        for (int l = plan.nlevels - 1; l >= 0; --l) {
-            int64_t first = plan.leaf_level_start[l];
-            item_lstart[l] = std::lower_bound(il.begin(), il.end(), (int32_t)first) - il.begin();
-        }
         item_leaf.upload(il);
         item_t0.upload(it);
         item_leaf_h = il;
@@ -1501,7 +1495,8 @@ struct Evaluator final : EvaluatorBase {
 
     NearArgs near_args(const P2pItems& it, int near, int mode, const double* q, double* fphi, double* fg, double* ophi,
                        double* og, double kre = 0.0, double kim = 0.0) const {
-        return NearArgs{dp, it, m, near, mode, spos.as<double4>(), q, tpos.as<double4>(), fphi, fg, ophi, og, kre, kim};
+        return NearArgs{dp, it, m, near, mode, spos.as<double4>(), q, tpos.as<double4>(), fphi, fg, ophi, og, kre, kim,
+                        num_sms};
     }
 
     // ---- the Helmholtz FMM (real k): complex expansions as row pairs, per-level tables ----
@@ -1566,6 +1561,7 @@ struct Evaluator final : EvaluatorBase {
                 if (kMixed) hq64.alloc(sizeof(double2) * (size_t)m * (dp.nsrc + 1));
             }
             const size_t smem = hh_expand_smem<P>(true, m);
+            // (the charges are staged 64 vectors at a time; the limit is the one callers know)
             if (sizeof(double) * 64 * (NC + (size_t)m) > 227 * 1024)
                 throw Failure(FMMGPU_UNSUPPORTED, "too many charge vectors a pass for P2L");
             CUDA_TRY(cudaFuncSetAttribute(hh_expand_kernel<P, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1746,7 +1742,7 @@ struct Evaluator final : EvaluatorBase {
                 dp, hh.lv, 0, (int64_t)plan.nleaves(), nullptr, m, spos.as<T4>(), hq.as<Cplx<T>>(), hM);
         upward<true>(hh.m2m.as<T>(), (int64_t)(8 * set), hh.Yo.as<T>(), hM);
         // M2L products of every level (their tables are per level): the mixed form on the
-        // tensor cores in one launch over every level, f64 on the SIMT GEMM level by level
+        // tensor cores in one launch over every level, f64 (gemm) level by level
         if constexpr (kHhTensor) {
             if (hh.tc_ntiles) {
                 const unsigned grid = (unsigned)std::min<int64_t>(hh.tc_ntiles, num_sms);

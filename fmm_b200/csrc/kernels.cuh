@@ -642,7 +642,8 @@ __global__ void __launch_bounds__(128, 4) local_reduce4_kernel(DevPlan plan, int
 }
 
 // ---------------------------------------------------------------------------------
-// Dense M2L as batched GEMM, SIMT form (f64 path): the V pairs of every level are
+// Dense translations as batched GEMM, SIMT form (f32: M2M and L2L of wide levels and the M2L path
+// without tensor cores; f64: the complex form above p = 8): the V pairs of every level are
 // grouped by offset index d (fmm-kernels/src/translate.rs:61-74 batches them the same
 // way); a block takes a tile of up to 64 pairs of one offset, stages A_d (column-major,
 // so row k of the staged array holds column k) and the tile's source multipoles in

@@ -212,6 +212,7 @@ struct NearArgs {
     const double4* tpos;
     double *far_phi, *far_g, *out_phi, *out_g;
     double k_re, k_im;  // the physical wavenumber
+    int num_sms;        // of the device
 };
 
 constexpr int kNearFlush = 64;    // sources a flush

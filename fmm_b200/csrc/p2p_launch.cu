@@ -38,13 +38,13 @@ void launch_p2p_st(const P2pStArgs& a, int warps, int ks, unsigned grid, cudaStr
 
 namespace {
 // Warps an item: 8, 4 or 2 while the items alone would leave most of an SM's schedulers
-// without a warp (148 SMs hold about eight of the kernel's warps each to be busy), else a
-// warp an item.  The floats are the same either way.
+// without a warp (an SM wants about eight of the kernel's warps to be busy), else a warp an
+// item.  The floats are the same either way.
 template <class PK>
 void launch_near(const NearArgs& a, cudaStream_t s) {
     const int64_t n = a.items.count;
     const size_t stage = sizeof(double) * near_stage_doubles<PK>() * kNearFlush;
-    const int w = n <= 2 * 148 ? 8 : n <= 4 * 148 ? 4 : n <= 8 * 148 ? 2 : 1;
+    const int w = n <= 2 * a.num_sms ? 8 : n <= 4 * a.num_sms ? 4 : n <= 8 * a.num_sms ? 2 : 1;
     if (w > 1)
         near_f64_kernel<PK, true><<<(unsigned)n, 32 * w, w * stage, s>>>(a);
     else
