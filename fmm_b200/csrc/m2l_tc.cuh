@@ -439,7 +439,8 @@ __global__ void __launch_bounds__(32 * kTcWarps, 1) m2l_tc_kernel(const int32_t*
             // bound the kernel more than any one role's work: without its conversions a sphere of
             // 1e6 points at p = 8 took 0.187 instead of 0.207 ms, without gathers, conversions and
             // stores 0.170; with this and the tiles' places read ahead 0.199, and the M2L of 4e6
-            // points 0.74 -> 0.66, of a batch with 16 vectors at p = 6 5.0 -> 4.5.)
+            // points 0.74 -> 0.66, of a batch with 16 vectors at p = 6 5.0 -> 4.5; a low part that keeps
+            // NaN, one more operation a value, 0.68 and 4.65.)
 #pragma unroll
             for (int g0 = 0; g0 < CV::STEPS; g0 += CV::N)
 #pragma unroll
