@@ -1560,7 +1560,9 @@ struct Evaluator final : EvaluatorBase {
                 hq.alloc(sizeof(Cplx<T>) * (size_t)m * (dp.nsrc + 1));
                 if (kMixed) hq64.alloc(sizeof(double2) * (size_t)m * (dp.nsrc + 1));
             }
-            const size_t smem = hh_expand_smem<P>(true, m);
+            // the most any handle asks for: the attribute is the kernel's, not the handle's, and a
+            // handle of fewer vectors must not lower it under another
+            const size_t smem = hh_expand_smem<P>(true, kHhVectors);
             // (the charges are staged 64 vectors at a time; the limit is the one callers know)
             if (sizeof(double) * 64 * (NC + (size_t)m) > 227 * 1024)
                 throw Failure(FMMGPU_UNSUPPORTED, "too many charge vectors a pass for P2L");

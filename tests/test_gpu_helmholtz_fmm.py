@@ -127,3 +127,20 @@ def test_local_expansions_keep_their_precision(p):
     want = (1 / scale).astype(float)
     assert np.sqrt((err[far] ** 2).sum() / (want[far] ** 2).sum()) < 2.9e-16
     fmm.close()
+
+
+@pytest.mark.parametrize("precision", ["f64", "mixed"])
+def test_handles_of_few_and_many_vectors_side_by_side(cloud, precision):
+    """The leaf sums' shared memory grows with the vectors: a handle of one vector set up after one of
+    many leaves the other's launches as they were."""
+    x, q = cloud
+    b = F.FmmBuilder(9).max_points_per_leaf(30).precision(precision)
+    qs = np.stack([q * (v + 1.0) for v in range(12)], axis=1)
+    many = b.vectors(12).build(x)
+    want = many.helmholtz_evaluate(4.0, qs).potential
+    one = b.vectors(1).build(x)
+    one.helmholtz_evaluate(4.0, q)
+    got = many.helmholtz_evaluate(4.0, qs).potential
+    assert np.array_equal(got, want)
+    one.close()
+    many.close()
